@@ -39,7 +39,7 @@ __device__ __forceinline__ R tvdb_face(R mm, R mc, R rm, R rc)
     if constexpr (EX)
         return (mm + mc) / (rm + rc);
     else
-        return fast_div(r_add(mm, mc), r_add(rm, rc));
+        return r_mul(r_add(mm, mc), fast_rcp(r_add(rm, rc)));
 }
 
 // 1-2-1 smoothing of the face velocity (C/advectbyzxA1.c:36-41): vm, v, vp at i-1, i, i+1.
@@ -112,8 +112,7 @@ __device__ __forceinline__ R tvdb_flux(R vbm, R vb0, R vbp, R vbpp, R vh, R dt)
         const R dp = r_sub(vbp, up ? vb0 : vbpp);
         const R dm = r_sub(vb0, up ? vbm : vbp);
         const R p = r_mul(dm, dp);
-        const R dw = (p > R(0)) ? fast_div(p, r_add(dm, dp)) : R(0);
-        return r_mul(r_add(w, dw), dt);
+        return r_mul(fma_if_pos(p, p, fast_rcp(r_add(dm, dp)), w), dt);
     }
 }
 

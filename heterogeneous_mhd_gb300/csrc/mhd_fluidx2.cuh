@@ -278,9 +278,33 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
             }
         }
     };
+    // x sweep: the field goes back over this thread's own cells of the staged
+    // b of plane k+1, which nobody else reads, so the second stage reads three
+    // values a cell instead of nine and does not build it again
+    R* const fown = (AX == 0) ? sbk + (size_t)lp * SB + (size_t)i0 * 3 : nullptr;
+    auto keep_f = [&](const R (&f)[C][3]) {
+        R ff[C * 3];
+#pragma unroll
+        for (int m = 0; m < C; m++)
+#pragma unroll
+            for (int s = 0; s < 3; s++)
+                ff[3 * m + s] = f[m][s];
+        sts_chunk<R, C * 3>(fown, ff);
+    };
+    auto again_f = [&](R (&f)[C][3]) {
+        R ff[C * 3];
+        lds_chunk<R, C * 3>(fown, ff);
+#pragma unroll
+        for (int m = 0; m < C; m++)
+#pragma unroll
+            for (int s = 0; s < 3; s++)
+                f[m][s] = ff[3 * m + s];
+    };
     R q[C][5], f[C][3];
     load_q(q);
     load_f(f);
+    if constexpr (AX == 0)
+        keep_f(f);
 
     // ---- stage 1 (C/tvd1.c:33-49)
     R fr[C][5], gl[C][5];  // fr = c*wr, gl = c*wl (so fl(i) = gl(i+1))
@@ -343,7 +367,10 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
     // ---- stage 2 (C/tvd1.c:51-116)
     {
         R v[C][5], cmax = R(0);
-        load_f(f);
+        if constexpr (AX == 0)
+            again_f(f);
+        else
+            load_f(f);
 #pragma unroll
         for (int m = 0; m < C; m++) {
             R ci;
@@ -404,25 +431,22 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
             for (int s = 0; s < 5; s++) {
                 const R dmn = (m + 1 < C) ? dm[m + 1][s] : xr[s];
                 const R dln = (m + 1 < C) ? dl[m + 1][s] : xr[5 + s];
-                R dfr, dfl;
-                if constexpr (EX) {
-                    dfr = vanleer<R, EX>(dmn, dm[m][s]);
-                    dfl = vanleer<R, EX>(dln, dl[m][s]);
-                } else {
-                    // branch-free: the quotient is computed for every cell and selected.
-                    // With a = A/2, b = B/2: 2ab / (a + b) = AB / (A + B), and every
-                    // factor dropped is a power of two, so the value is the halved form's.
-                    const R pr = dmn * dm[m][s], pl = dln * dl[m][s];
-                    const R qr = fast_div(pr, dmn + dm[m][s]), ql = fast_div(pl, dln + dl[m][s]);
-                    dfr = (pr > R(0)) ? qr : R(0);
-                    dfl = (pl > R(0)) ? ql : R(0);
-                }
                 const R gn = (m + 1 < C) ? gl[m + 1][s] : gln[s];
-                if constexpr (EX)
+                if constexpr (EX) {
+                    const R dfr = vanleer<R, EX>(dmn, dm[m][s]);
+                    const R dfl = vanleer<R, EX>(dln, dl[m][s]);
                     flux[m][s] = lin<R, EX>(R(0.5), lin<R, EX>(R(1), fr[m][s], R(-1), gn), R(0.5),
                                             lin<R, EX>(R(1), dfr, R(-1), dfl));
-                else  // undivided (2 flux), the half goes into the step below
-                    flux[m][s] = (fr[m][s] - gn) + (dfr - dfl);
+                } else {
+                    // branch-free: the reciprocal is taken for every cell.  With a = A/2,
+                    // b = B/2: 2ab / (a + b) = AB / (A + B), and every factor dropped is a
+                    // power of two.  The limited differences go straight into the flux,
+                    // which is kept undivided (2 flux; the half goes into the step below).
+                    const R pr = dmn * dm[m][s], pl = dln * dl[m][s];
+                    R t = fr[m][s] - gn;
+                    t = fma_if_pos(pr, pr, fast_rcp(dmn + dm[m][s]), t);
+                    flux[m][s] = fma_if_pos(pl, -pl, fast_rcp(dln + dl[m][s]), t);
+                }
             }
     }
     {
