@@ -355,7 +355,7 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
             }
         R fprev[5];
         g.template shift<5>(flux[C - 1], fprev, -1, seam, 1);
-        const R hdt = EX ? R(W(-1.0) * W(dt) / W(2.0)) : R(-0.25) * dt;
+        const R hdt = EX ? R(-0.5) * dt : R(-0.25) * dt;
 #pragma unroll
         for (int m = 0; m < C; m++)
 #pragma unroll
@@ -452,7 +452,7 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
     {
         R fprev[5];
         g.template shift<5>(flux[C - 1], fprev, -1, seam, 1);
-        const R mdt = EX ? R(W(-1.0) * W(dt)) : R(-0.5) * dt;
+        const R mdt = EX ? -dt : R(-0.5) * dt;
         R of[C * 5];
         load_q(q);
 #pragma unroll

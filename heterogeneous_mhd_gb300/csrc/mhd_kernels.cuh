@@ -330,8 +330,7 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
     }
     __syncthreads();
     {
-        using W = wide_t<R, EX>;
-        const R hdt = R(W(-1.0) * W(dt) / W(2.0));
+        const R hdt = R(-0.5) * dt;  // -1.0 * dt / 2.0 in double: exact
 #pragma unroll
         for (int s = 0; s < 5; s++)
             u1[s] = lin<R, EX>(R(1), q[s], hdt, lin<R, EX>(R(1), flux[s], R(-1), xb[5 * mem + s]));
@@ -379,8 +378,7 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
     }
     __syncthreads();
     {
-        using W = wide_t<R, EX>;
-        const R mdt = R(W(-1.0) * W(dt));
+        const R mdt = -dt;
 #pragma unroll
         for (int s = 0; s < 5; s++) {
             const R un = lin<R, EX>(R(1), q[s], mdt, lin<R, EX>(R(1), flux[s], R(-1), xa[5 * mem + s]));
@@ -521,11 +519,7 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
         const int r = it / n, i = it - r * n;
         const int ip = (i + 1 == n) ? 0 : i + 1, im = (i == 0) ? n - 1 : i - 1;
         const R* row = VR + r * n;
-        R vg;
-        if constexpr (EX)
-            vg = R((W(row[im] + row[ip]) + W(2.0) * W(row[i])) / W(4.0));
-        else
-            vg = ((row[im] + row[ip]) + R(2) * row[i]) * R(0.25);
+        const R vg = tvdb_smooth<R, EX>(row[im], row[i], row[ip]);
         VG[it] = vg;
         T2[it] = BV[it] * vg;
     }
@@ -543,12 +537,7 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
         const int r = it / n, i = it - r * n;
         const int im = (i == 0) ? n - 1 : i - 1;
-        R b1;
-        if constexpr (EX)
-            b1 = R(W(BV[it]) - W((F1[it] - F1[r * n + im]) * dt) / W(2.0));
-        else
-            b1 = BV[it] - (F1[it] - F1[r * n + im]) * dt * R(0.5);
-        T2[it] = VG[it] * b1;
+        T2[it] = tvdb_prod<R, EX>(VG[it], tvdb_half<R, EX>(BV[it], F1[it], F1[r * n + im], dt));
     }
     __syncthreads();
     // Phase 5: limited upwind flux (C/tvdb.c:54-78).
@@ -558,18 +547,7 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
         const int ipp = (ip + 1 == n) ? 0 : ip + 1;
         const int im = (i == 0) ? n - 1 : i - 1;
         const R* vb = T2 + r * n;
-        R w, wp, wm;
-        if (VH[it] > R(0)) {
-            w = vb[i];
-            wp = R(W(vb[ip] - w) / W(2.0));
-            wm = R(W(w - vb[im]) / W(2.0));
-        } else {
-            w = vb[ip];
-            wp = R(W(w - vb[ipp]) / W(2.0));
-            wm = R(W(vb[i] - w) / W(2.0));
-        }
-        const R dw = vanleer<R, EX>(wm, wp);
-        FX[it] = (w + dw) * dt;
+        FX[it] = tvdb_flux<R, EX>(vb[im], vb[i], vb[ip], vb[ipp], VH[it], dt);
     }
     __syncthreads();
     // Phase 6: b - (flux - flux(i-1)) (C/tvdb.c:79-88) into VR.

@@ -90,6 +90,126 @@ __device__ __forceinline__ double fma_if_pos(double p, double x, double r, doubl
     return (p > 0.0) ? fma(x, r, t) : t;
 }
 
+// ------------------------------------------- EXACT in FP32 without FP64
+//
+// The reference is C on float data whose double literals promote a few
+// sub-expressions to double before they are rounded back to float.  This GPU
+// runs FP64 at 1/60 of its FP32 rate (measured: 0.017 against 1.05 warp
+// instructions per clock and scheduler), so those promotions were nearly all
+// of the EXACT kernels' time.  Each is evaluated as an unevaluated sum of two
+// floats instead (error-free sums and products: Dekker 1971, Knuth TAOCP 4.2.2)
+// whose distance from the double expression is bounded, and rounded with
+// Ziv's test (ACM TOMS 17, 1991): if both ends of the interval round to the
+// same float, the double expression does too.  Where they do not (about one
+// value in 2^16), or where a range condition of the bound fails (tiny or huge
+// operands, infinities, NaN), the double expression itself is evaluated.
+//
+// Two EXACT 96^3 steps: 6.07 ms with the double sub-expressions (fluidx 340,
+// advectbyzx 148 us per launch), 1.15 ms with these; same bits.
+
+// sum + lo with |error| <= err around hi + lo: true if the rounding is certain
+__device__ __forceinline__ bool ziv_round(float hi, float lo, float err, float& r)
+{
+    r = __fadd_rn(hi, __fsub_rn(lo, err));
+    return r == __fadd_rn(hi, __fadd_rn(lo, err));
+}
+
+// s + e = a + b exactly (Knuth)
+__device__ __forceinline__ void two_sum(float a, float b, float& s, float& e)
+{
+    s = __fadd_rn(a, b);
+    const float t = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+}
+
+// float(2ab / (a + b)) with the product and the quotient in double, for a b > 0
+static __device__ __noinline__ float vanleer_wide(float a, float b) { return float(2.0 * double(a) * double(b) / double(a + b)); }
+
+__device__ __forceinline__ float vanleer_exact(float a, float b)
+{
+    float r = 0.f;
+    if (__fmul_rn(a, b) > 0.f) {
+        const float a2 = __fadd_rn(a, a), s = __fadd_rn(a, b);
+        const float ph = __fmul_rn(a2, b), pl = __fmaf_rn(a2, b, -ph);  // 2ab = ph + pl
+        const float y = fast_rcp(s), q = __fmul_rn(ph, y);              // q within 2^-21.6 of the quotient
+        const float e = __fmul_rn(__fadd_rn(__fmaf_rn(-q, s, ph), pl), y);
+        // |q + e - quotient| <= 2^-42.6 |q| (the residual's, the product's and y's errors
+        // on a correction of at most 2^-21.4 |q|), 2^-45 for lo -+ err, 2^-53 for the double
+        const bool sure = ziv_round(q, e, fabsf(q) * 0x1p-41f, r);
+        // the product's and the residual's low parts are exact above 2^-100
+        if (!(sure && ph > 0x1p-100f && fabsf(q) > 0x1p-80f && fabsf(s) < 0x1p100f))
+            r = vanleer_wide(a, b);
+    }
+    return r;
+}
+
+constexpr float kGammaF = float(5.0 / 3.0);
+constexpr float kGm1F = float(double(kGammaF) - 1.0), kHalf2mgF = float((2.0 - double(kGammaF)) / 2.0);
+static_assert(double(kGm1F) == double(kGammaF) - 1.0 && double(kHalf2mgF) == (2.0 - double(kGammaF)) / 2.0,
+              "gamma - 1 and (2 - gamma) / 2 are floats");
+
+// float((e - h/2)(gamma - 1) + (2 - gamma) bb / 2) in double
+static __device__ __noinline__ float total_pressure_wide(float e, float h, float bb)
+{
+    return float((double(e) - double(h) / 2.0) * (double(kGammaF) - 1.0) + (2.0 - double(kGammaF)) * double(bb) / 2.0);
+}
+
+__device__ __forceinline__ float total_pressure_exact(float e, float h, float bb)
+{
+    float t, te, s, se, r;
+    two_sum(e, __fmul_rn(-0.5f, h), t, te);
+    const float p = __fmul_rn(t, kGm1F), pe = __fmaf_rn(te, kGm1F, __fmaf_rn(t, kGm1F, -p));
+    const float c = __fmul_rn(kHalf2mgF, bb), ce = __fmaf_rn(kHalf2mgF, bb, -c);
+    two_sum(p, c, s, se);
+    // three roundings of terms of at most 2^-23 (|p| + |c|): within 2^-45.4 of it
+    const float m = __fadd_rn(fabsf(p), fabsf(c));
+    const bool sure = ziv_round(s, __fadd_rn(se, __fadd_rn(pe, ce)), m * 0x1p-44f, r);
+    if (!(sure && m > 0x1p-90f && m < 0x1p100f))
+        r = total_pressure_wide(e, h, bb);
+    return r;
+}
+
+// float(a + sqrt(t)) in double, for a >= 0 and t >= 0
+static __device__ __noinline__ float add_sqrt_wide(float a, float t) { return float(double(a) + sqrt(double(t))); }
+
+__device__ __forceinline__ float add_sqrt_exact(float a, float t)
+{
+    float s, se, r;
+    const float s0 = fast_sqrt(t);  // within 2^-22: with the correction's own error 2^-42.5 of s0
+    const float corr = __fmul_rn(__fmaf_rn(-s0, s0, t), __fmul_rn(0.5f, fast_rcp(s0)));
+    two_sum(a, s0, s, se);
+    const bool sure = ziv_round(s, __fadd_rn(se, corr), s * 0x1p-41f, r);
+    if (!(sure && s0 > 0x1p-40f && s < 0x1p60f))
+        r = add_sqrt_wide(a, t);
+    return r;
+}
+
+// float(v + sqrt(|2 bb + g| / rho)) in double, for v >= 0
+static __device__ __noinline__ float cfl_wide(float v, float bb, float g, float rho)
+{
+    return float(double(v) + sqrt(fabs(double(bb) * 2.0 + double(g)) / double(rho)));
+}
+
+__device__ __forceinline__ float cfl_exact(float v, float bb, float g, float rho)
+{
+    float nh, nl, s, se, r;
+    two_sum(__fadd_rn(bb, bb), g, nh, nl);
+    if (nh < 0.f) {
+        nh = -nh;
+        nl = -nl;
+    }
+    const float y = fast_rcp(rho), q = __fmul_rn(nh, y);
+    const float e = __fmul_rn(__fadd_rn(__fmaf_rn(-q, rho, nh), nl), y);
+    const float s0 = fast_sqrt(q);
+    const float corr = __fmul_rn(__fadd_rn(__fmaf_rn(-s0, s0, q), e), __fmul_rn(0.5f, fast_rcp(s0)));
+    two_sum(v, s0, s, se);
+    // the quotient within 2^-42.6, the root within half of that and 2^-44 (corr up to 2^-21)
+    const bool sure = ziv_round(s, __fadd_rn(se, corr), s * 0x1p-40f, r);
+    if (!(sure && q > 0x1p-60f && q < 0x1p60f && rho > 0x1p-40f && rho < 0x1p40f && s < 0x1p60f))
+        r = cfl_wide(v, bb, g, rho);
+    return r;
+}
+
 // abXYc_matrix2D with c = 0 (C/includefunc_spu.h:73-84): a*X + b*Y + 0.
 template <typename R, bool EX>
 __device__ __forceinline__ R lin(R a, R x, R b, R y)
@@ -116,7 +236,9 @@ template <typename R, bool EX>
 __device__ __forceinline__ R vanleer(R a, R b)
 {
     using W = wide_t<R, EX>;
-    if constexpr (EX) {
+    if constexpr (EX && sizeof(R) == 4) {
+        return vanleer_exact(a, b);
+    } else if constexpr (EX) {
         R r = R(0);
         if (a * b > R(0))
             r = R(W(2.0) * W(a) * W(b) / W(a + b));
@@ -139,15 +261,26 @@ __device__ __forceinline__ void cell_flux(const R q[5], const R f[3], R v[5], R&
         R vx = q[1] / q[0];
         R mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
         R bb = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
-        R ps = R((W(q[4]) - W(mm / q[0]) / W(2.0)) * (W(gamma) - W(1.0)) +
-                 (W(2.0) - W(gamma)) * W(bb) / W(2.0));
+        R ps;
+        if constexpr (sizeof(R) == 4)
+            ps = total_pressure_exact(q[4], mm / q[0], bb);
+        else
+            ps = R((W(q[4]) - W(mm / q[0]) / W(2.0)) * (W(gamma) - W(1.0)) +
+                   (W(2.0) - W(gamma)) * W(bb) / W(2.0));
         v[0] = q[1];
         v[1] = q[1] * vx + ps - f[0] * f[0];
         v[2] = q[2] * vx - f[1] * f[0];
         v[3] = q[3] * vx - f[2] * f[0];
         v[4] = (q[4] + ps) * vx - f[0] * (f[0] * q[1] + f[1] * q[2] + f[2] * q[3]) / q[0];
-        R p = R(W(ps) - W(bb) / W(2.0));
-        ci = R(fabs(W(vx)) + sqrt(fabs(W((bb + gamma * p) / q[0]))));
+        if constexpr (sizeof(R) == 4) {
+            // a difference of two floats rounds alike with and without the double between
+            // (53 >= 2 * 24 + 2), so one fused step gives it
+            const R p = __fmaf_rn(-0.5f, bb, ps);
+            ci = add_sqrt_exact(fabsf(vx), fabsf((bb + gamma * p) / q[0]));
+        } else {
+            R p = R(W(ps) - W(bb) / W(2.0));
+            ci = R(fabs(W(vx)) + sqrt(fabs(W((bb + gamma * p) / q[0]))));
+        }
     } else {
         const R ri = fast_rcp(q[0]);
         const R vx = q[1] * ri;
@@ -198,12 +331,16 @@ __device__ __forceinline__ R cfl_speed(const R q[5], const R f[3])
     using W = wide_t<R, EX>;
     const R gamma = R(5.0 / 3.0);
     if constexpr (EX) {
-        R t1 = R(fabs(W(q[1] / q[0])));
-        R t2 = R(fabs(W(q[2] / q[0])));
-        R t3 = R(fabs(W(q[3] / q[0])));
+        R t1 = rabs(q[1] / q[0]);
+        R t2 = rabs(q[2] / q[0]);
+        R t3 = rabs(q[3] / q[0]);
         R v = max3(t1, t2, t3);
         R mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
         R bb = f[0] * f[0] + f[1] * f[1] + f[2] * f[2];
+        if constexpr (sizeof(R) == 4) {
+            const R ps = total_pressure_exact(q[4], mm / q[0], bb);
+            return cfl_exact(v, bb, gamma * __fmaf_rn(-0.5f, bb, ps), q[0]);
+        }
         R ps = R((W(q[4]) - W(mm / q[0]) / W(2.0)) * (W(gamma) - W(1.0)) +
                  (W(2.0) - W(gamma)) * W(bb) / W(2.0));
         R p = R(W(ps) - W(bb) / W(2.0));
@@ -217,6 +354,122 @@ __device__ __forceinline__ R cfl_speed(const R q[5], const R f[3])
         const R p = ps - R(0.5) * bb;
         return v + fast_sqrt(rabs(bb * R(2) + gamma * p) * ri);
     }
+}
+
+// Per-cell steps of tvdb, shared by every advectbyzx kernel.  EXACT: the
+// reference's expressions (compiled without contraction).  FAST: every
+// rounding is explicit (__fadd_rn, __fmul_rn and __fmaf_rn are never
+// contracted), so all kernels compute the same bits whatever the compiler
+// does around the calls.
+__device__ __forceinline__ float r_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double r_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ double r_sub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ float r_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double r_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float r_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double r_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// Raw face velocity (C/advectbyzxA1.c:34, C/advectbyzxB1.c:34) from m_x and
+// rho of the pencil below (m) and the current one (c).
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_face(R mm, R mc, R rm, R rc)
+{
+    if constexpr (EX)
+        return (mm + mc) / (rm + rc);
+    else
+        return r_mul(r_add(mm, mc), fast_rcp(r_add(rm, rc)));
+}
+
+// 1-2-1 smoothing of the face velocity (C/advectbyzxA1.c:36-41): vm, v, vp at i-1, i, i+1.
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_smooth(R vm, R v, R vp)
+{
+    using W = wide_t<R, EX>;
+    if constexpr (EX && sizeof(R) == 4) {
+        // the sum of two floats rounds alike with and without the double between, and the
+        // quarter is exact unless it is subnormal
+        const R f = vm + vp, t = r_fma(R(2), v, f);
+        return (t == R(0) || fabsf(t) > 0x1p-120f) ? t * R(0.25) : R((W(f) + W(2.0) * W(v)) / W(4.0));
+    } else if constexpr (EX)
+        return R((W(vm + vp) + W(2.0) * W(v)) / W(4.0));
+    else
+        return r_mul(r_fma(R(2), v, r_add(vm, vp)), R(0.25));
+}
+
+// b vg (C/tvdb.c:31-34), vg b1 (C/tvdb.c:55-60)
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_prod(R x, R y)
+{
+    if constexpr (EX)
+        return x * y;
+    else
+        return r_mul(x, y);
+}
+
+// vh = (vg(i) + vg(i+1)) / 2 in the abXYc form (C/tvdb.c:25-29)
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_vh(R vg, R vgn)
+{
+    if constexpr (EX)
+        return lin<R, EX>(R(0.5), vg, R(0.5), vgn);
+    else
+        return r_fma(R(0.5), vg, r_mul(R(0.5), vgn));
+}
+
+// Half step b1 = b - (f1(i) - f1(i-1)) dt / 2 (C/tvdb.c:41-47).
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_half(R bv, R f1, R fm, R dt)
+{
+    using W = wide_t<R, EX>;
+    if constexpr (EX && sizeof(R) == 4)  // bv - x / 2 rounded once: the double between does not change it
+        return r_fma(R(-0.5), (f1 - fm) * dt, bv);
+    else if constexpr (EX)
+        return R(W(bv) - W((f1 - fm) * dt) / W(2.0));
+    else  // dt / 2 is loop-invariant: one fused multiply-add per cell
+        return r_fma(r_sub(fm, f1), r_mul(dt, R(0.5)), bv);
+}
+
+// Limited upwind flux times dt at i+1/2 (C/tvdb.c:54-78) from vb = vg b1 at
+// i-1, i, i+1, i+2 and the sign of vh(i).
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_flux(R vbm, R vb0, R vbp, R vbpp, R vh, R dt)
+{
+    if constexpr (EX) {
+        // halves of differences: R(0.5) x rounds as the double quotient by 2.0 does
+        R w, wp, wm;
+        if (vh > R(0)) {
+            w = vb0;
+            wp = R(0.5) * (vbp - w);
+            wm = R(0.5) * (w - vbm);
+        } else {
+            w = vbp;
+            wp = R(0.5) * (w - vbpp);
+            wm = R(0.5) * (vb0 - w);
+        }
+        const R dw = vanleer<R, EX>(wm, wp);
+        return (w + dw) * dt;
+    } else {
+        // The same differences with the operands selected (no branch), and the
+        // limiter on the undivided differences: with wm = dm/2, wp = dp/2,
+        // 2 wm wp / (wm + wp) = dm dp / (dm + dp).
+        const bool up = vh > R(0);
+        const R w = up ? vb0 : vbp;
+        const R dp = r_sub(vbp, up ? vb0 : vbpp);
+        const R dm = r_sub(vb0, up ? vbm : vbp);
+        const R p = r_mul(dm, dp);
+        return r_mul(fma_if_pos(p, p, fast_rcp(r_add(dm, dp)), w), dt);
+    }
+}
+
+// Advected field b - (flux(i) - flux(i-1)) (C/tvdb.c:79-88)
+template <typename R, bool EX>
+__device__ __forceinline__ R tvdb_new(R bv, R flux, R fm)
+{
+    if constexpr (EX)
+        return bv - (flux - fm);
+    else
+        return r_sub(bv, r_sub(flux, fm));
 }
 
 }  // namespace mhd

@@ -249,3 +249,32 @@ def test_empty_grid(mhd, cuda):
     uo = np.full(5, 3, dtype=np.float32)
     mhd.fluidx(uo, b, 0, 4, 4, 0.1, u, b)
     assert (uo == 3).all()
+
+
+@pytest.mark.parametrize("shape", [(32, 8, 4), (96, 6, 3), (20, 5, 3), (256, 4, 2)])
+@pytest.mark.parametrize("lo,hi", [(-6, 2), (-45, 6), (-70, 20)])
+def test_exact_ops_wide_magnitudes_vs_oracle(shape, lo, hi, mhd, cuda, oracle32):
+    """EXACT evaluates the reference's double sub-expressions as certified sums of two
+    floats, with the double expression where the rounding is not certain or a range
+    condition fails: momenta, energies and fields of 2^lo .. 2^hi (signs and exact zeros
+    mixed in) around ordinary densities, bit for bit against the oracle."""
+    nx, ny, nz = shape
+    rng = np.random.default_rng(nx * 1000 + 7 * hi - lo)
+    nc = nx * ny * nz
+    u = (rng.standard_normal((nc, 5)) * 2.0 ** rng.uniform(lo, hi, (nc, 5))).astype(np.float32)
+    u[:, 0] = 2.0 ** rng.uniform(-3, 3, nc)
+    u[rng.random((nc, 5)) < 0.05] = 0
+    u[:, 0] = np.where(u[:, 0] == 0, 1, u[:, 0])
+    b = (rng.standard_normal((nc, 3)) * 2.0 ** rng.uniform(lo, hi, (nc, 3))).astype(np.float32)
+    b[rng.random((nc, 3)) < 0.05] = 0
+    u, b = u.ravel(), b.ravel()
+    bin_ = (b * np.float32(0.75)).astype(np.float32)
+    uo, bo = np.full_like(u, 7), bin_.copy()
+    oracle32.fluidx(uo, b.copy(), nx, ny, nz, DT, u.copy(), b.copy())
+    oracle32.advectbyzx(u.copy(), bo, nx, ny, nz, DT, u.copy(), b.copy())
+    ref_cfl = oracle32.calcfl(u, b, nx, ny, nz)
+    with mhd.Context(1, 1, 1, exact=True) as ctx:
+        out = run_ops(mhd, cuda, ctx, u, b, bin_, nx, ny, nz)
+    assert bitwise_equal(out["fluidx_u"], uo)
+    assert bitwise_equal(out["advect_b"], bo)
+    assert out["calcfl"][0] == np.float32(ref_cfl)
