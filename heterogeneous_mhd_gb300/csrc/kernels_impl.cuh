@@ -3,8 +3,8 @@
 //
 // Each operator has a register-resident kernel for the common pencil lengths
 // (fluidx: n = 4T with T in {8..128} or 3T with T in {16..128}; advectbyzx:
-// n = 8T, T in {4..64} or 6T, T in {8..64}; transposes: full 32x32 tiles, or
-// 16x16 tiles for edges that are multiples of 16) and a general kernel for
+// n = 8T, T in {4..64} or 6T, T in {8..64}; transposes: bulk-TMA tiles of 32x32 or
+// 16x16 cells for edges that are multiples of 16) and a general kernel for
 // every other shape.  FP64 uses the general kernels.  The batch's work-list
 // launches (one launch per operator over several size classes) are at the end.
 #include "mhd_advect2.cuh"
@@ -16,7 +16,6 @@
 #include "mhd_launch.h"
 #include "mhd_multi.cuh"
 #include "mhd_tmap.h"
-#include "mhd_transpose2.cuh"
 #include "mhd_transpose3.cuh"
 
 namespace mhd {
@@ -25,31 +24,6 @@ namespace MHD_SET_NAME {
 using R = MHD_REAL;
 constexpr bool EX = MHD_EXACT;
 constexpr bool kV2 = (sizeof(R) == 4);
-
-// Raise a kernel's dynamic shared-memory limit to the device's opt-in maximum
-// minus its static shared memory (once per kernel).  Kernels that stage all
-// their input by TMA ask for the largest shared-memory carveout (they do not
-// use L1 for data), so residency is set by registers and shared memory only.
-template <typename K>
-static cudaError_t allow_smem(K kernel, bool& done, bool tma_staged = false)
-{
-    if (done)
-        return cudaSuccess;
-    int dev = 0, optin = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess)
-        e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncAttributes fa{};
-    if (e == cudaSuccess)
-        e = cudaFuncGetAttributes(&fa, kernel);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
-    if (e == cudaSuccess && tma_staged)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (e == cudaSuccess)
-        done = true;
-    return e;
-}
 
 // devices whose occupancy figures the persistent launchers cache
 constexpr int kMaxOccDevices = 64;
@@ -165,6 +139,24 @@ static bool fluidx_range_ok(const FluidxArgs& a)
     return a.axis == 1 || plan_fluidx(a.nx, a.ny, a.use_tma != 0).C != 0;
 }
 
+// Every other pencil length, and unaligned arrays: FP32 the ragged engine
+// (mhd_ragged.cuh), FP64 one thread per cell (bound by the FP64 pipe).
+template <typename RR>
+static cudaError_t fluidx_any(const FluidxArgs& a, cudaStream_t s)
+{
+    if constexpr (sizeof(RR) == 4) {
+        return fluidx_ragged(a, EX, s);
+    } else {
+        static bool attr = false;
+        cudaError_t e = allow_smem(k_fluidx<RR, EX>, attr);
+        if (e != cudaSuccess)
+            return e;
+        dim3 grid(a.ny / a.P, a.nz, a.bs.count);
+        k_fluidx<RR, EX><<<grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx, a.P) * sizeof(RR), s>>>(a);
+        return cudaGetLastError();
+    }
+}
+
 static cudaError_t fluidx(const FluidxArgs& in, cudaStream_t s)
 {
     FluidxArgs a = in;
@@ -207,18 +199,14 @@ static cudaError_t fluidx(const FluidxArgs& in, cudaStream_t s)
             }
         }
     }
-    static bool attr = false;
-    cudaError_t e = allow_smem(k_fluidx<R, EX>, attr);
-    if (e != cudaSuccess)
-        return e;
-    dim3 grid(a.ny / a.P, a.nz, a.bs.count);
-    k_fluidx<R, EX><<<grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx, a.P) * sizeof(R), s>>>(a);
-    return cudaGetLastError();
+    return fluidx_any<R>(a, s);
 }
 
 static int fluidx_parts(int nx, int ny, int nz, int aligned)
 {
     const FxPlan p = plan_fluidx(nx, ny, aligned != 0);
+    if (kV2 && p.C == 0)
+        return rag_fluidx_parts(nx, ny, nz);
     return (ny / p.P) * nz;
 }
 
@@ -674,6 +662,8 @@ static cudaError_t advect(const AdvectArgs& in, cudaStream_t s)
             case 64: return launch_ad2<6, 64>(a, s);
             }
         }
+        if (rag_shape(a.nx, 2).C)
+            return advect_ragged(a, EX, s);
     }
     static bool attr = false;
     cudaError_t e = allow_smem(k_advect<R, EX>, attr);
@@ -714,18 +704,13 @@ static cudaError_t transpose(const TransposeArgs& a, cudaStream_t s)
                 k_transpose3<2, 16><<<grid, 256, 0, s>>>(a);
             return cudaGetLastError();
         }
-        if (a.nx % kT2 == 0 && na % kT2 == 0 && (al & 3) == 0) {
-            dim3 grid(a.nx / kT2, na / kT2, nb * a.bs.count);
-            if (a.axis == 1)
-                k_transpose2<1><<<grid, 256, 0, s>>>(a);
-            else
-                k_transpose2<2><<<grid, 256, 0, s>>>(a);
-            return cudaGetLastError();
-        }
     }
     constexpr int T = TTile<R>::E;
     dim3 grid((a.nx + T - 1) / T, (na + T - 1) / T, nb * a.bs.count);
-    k_transpose<R><<<grid, 256, 0, s>>>(a);
+    if (a.axis == 1)
+        k_transpose<1, R><<<grid, 256, 0, s>>>(a);
+    else
+        k_transpose<2, R><<<grid, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -783,20 +768,20 @@ static int fused_ok(int nx, int ny, int nz)
     return plan_fluidx_sweep(ny, nx, 1, p) && plan_fluidx_sweep(nz, nx, 1, p) && advect_ok(1) && advect_ok(2);
 }
 
-// nonzero if the x-sweep fluidx of this grid is k_fluidx2 (which writes the
-// (rho, m_x) side array when asked)
+// nonzero if the x-sweep fluidx of this grid writes the (rho, m_x) side array
+// when asked: every FP32 kernel does
 static int fluidx_writes_w(int nx, int ny, int nz, int aligned)
 {
-    (void)nz;
-    return kV2 && plan_fluidx(nx, ny, aligned != 0).C != 0;
+    (void)nx, (void)ny, (void)nz, (void)aligned;
+    return kV2;
 }
 
-// nonzero if the transpose of this grid is k_transpose3 (which writes the side
-// array when asked); nx, ny, nz are the input dims, the buffers 16-byte aligned
+// nonzero if the transpose of this grid writes the side array when asked:
+// every FP32 kernel does
 static int transpose_writes_w(int axis, int nx, int ny, int nz)
 {
-    const int na = (axis == 1) ? ny : nz;
-    return kV2 && nx % kT3 == 0 && na % kT3 == 0;
+    (void)axis, (void)nx, (void)ny, (void)nz;
+    return kV2;
 }
 
 // nonzero if the fused step's fluidx sweep along `axis` (1: y, 2: z) of this
@@ -984,9 +969,7 @@ static cudaError_t transpose_multi(const TransposeArgs* in, int nseg, cudaStream
             if (a.axis != axis || (axis != 1 && axis != 2) || (al & 15) != 0)
                 return cudaErrorInvalidValue;
             const int n = a.nx;
-            const int kind = (n % 32 == 0) ? 0 : ((n % 16 == 0) ? 2 : 1);
-            const int E = (kind == 0) ? 32 : ((kind == 2) ? 16 : TTile<float>::E);
-            const int g = (n + E - 1) / E;
+            const int kind = (n % 32 == 0) ? 0 : 2, E = (kind == 0) ? 32 : 16, g = n / E;  // multi_ok's edges
             m.a[i] = a;
             m.g[i] = SegGrid{(int)total, g, g, kind};
             total += (long long)g * g * n * a.bs.count;

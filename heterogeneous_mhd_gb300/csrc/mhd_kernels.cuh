@@ -609,33 +609,34 @@ struct TTile {
 };
 
 // transpose12 (C/transpose12.c:7-47) and transpose13 (C/transpose13.c:9-62):
-// out(a, ., i) = in(i, ., a) with the component permutation of each.  A CTA
-// moves a 32x32 tile of cells through shared memory so both the reads (rows
-// of x) and the writes (rows of the swapped axis) are contiguous.  Tiles at
-// the edges of grids that are not multiples of 32 are partial.
+// out(a, ., i) = in(i, ., a) with the component permutation of each, for any
+// edges (the bulk-TMA tiles of mhd_transpose3.cuh take multiples of 16 in FP32).
+// A CTA moves a tile of at most kTT x kTT cells through shared memory so both
+// the reads (rows of x) and the writes (rows of the swapped axis) are
+// contiguous; an edge is cut into equal tiles (72 into 24s, not 32 + 32 + 8).
 //
-// The body stages into su [kTT][kTT*5+1] and sb [kTT][kTT*3+1] and takes the
-// CTA's block coordinates `blk` (HwBlock and static arrays in k_transpose,
-// VBlock and dynamic shared memory in the work-list launch over several size
-// classes, mhd_multi.cuh).  With w_out (FP32) it also writes the first two
-// components of the output cells, the (rho, m_x) side array.
-template <typename R>
-__host__ __device__ constexpr size_t transpose_smem_bytes()
+// A warp owns whole rows on both sides: all of its loads are issued before its
+// shared stores (up to 32 in flight a lane), and a lane's source offsets inside
+// an output row are computed once.  Row strides of 5 kTT + 5 and 3 kTT + 3 words
+// put the 32 lanes of an output row on 32 banks.  Bound by memory latency at the
+// sizes it serves; 100 x 72 x 72 measured 31 us a launch when each output row was
+// written by the whole CTA with divisions per element, 14 us now (event pairs).
+//
+// With w_out (FP32) it also writes the first two components of the output
+// cells, the (rho, m_x) side array.
+template <int AXIS, typename R>
+__device__ __forceinline__ void transpose_tile(const TransposeArgs& a, R* su, R* sb, int z)
 {
-    return (size_t)TTile<R>::E * (TTile<R>::E * 8 + 2) * sizeof(R);
-}
-
-template <typename R, typename B>
-__device__ __forceinline__ void transpose_body(TransposeArgs a, R* su, R* sb, const B& blk)
-{
-    constexpr int kTT = TTile<R>::E;
-    constexpr int SU = kTT * 5 + 1, SB = kTT * 3 + 1;  // padded row strides
+    constexpr int E = TTile<R>::E, SU = 5 * E + 5, SB = 3 * E + 3;  // padded row strides
+    constexpr int QU = (5 * E + 31) / 32, QB = (3 * E + 31) / 32, QW = (2 * E + 31) / 32, RW = E / 8;
     const int nx = a.nx, ny = a.ny, nz = a.nz;
-    const int na = (a.axis == 1) ? ny : nz;  // extent of the swapped axis
-    const int nbz = (a.axis == 1) ? nz : ny;  // extent of the untouched axis
-    const int i0 = blk.x() * kTT, a0 = blk.y() * kTT, z = blk.z() % nbz;
-    select_box(a, blk.z() / nbz);
-    const int ti = min(kTT, nx - i0), ta = min(kTT, na - a0);
+    const int na = (AXIS == 1) ? ny : nz;  // extent of the swapped axis
+    const int ei = (nx + gridDim.x - 1) / gridDim.x, ea = (na + gridDim.y - 1) / gridDim.y;
+    const int i0 = blockIdx.x * ei, a0 = blockIdx.y * ea;
+    const int ti = min(ei, nx - i0), ta = min(ea, na - a0);
+    if (ti <= 0 || ta <= 0)  // the equal tiles before this one reach the edge
+        return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const R* uu = static_cast<const R*>(a.uu);
     const R* ub = static_cast<const R*>(a.ub);
     R* uo = static_cast<R*>(a.u_out);
@@ -643,49 +644,87 @@ __device__ __forceinline__ void transpose_body(TransposeArgs a, R* su, R* sb, co
     R* wo = static_cast<R*>(a.w_out);
 
     // input cell (i, a, z) for axis 1 is (i, j=a, k=z); for axis 2 it is (i, j=z, k=a)
-    const size_t rstride = (a.axis == 1) ? (size_t)nx : (size_t)nx * ny;  // cells between rows of a
-    const size_t cin0 = (a.axis == 1) ? (((size_t)z * ny + a0) * nx + i0) : (((size_t)a0 * ny + z) * nx + i0);
-    for (int e = threadIdx.x; e < ta * ti * 5; e += blockDim.x) {
-        const int r = e / (ti * 5), c = e - r * (ti * 5);
-        su[r * SU + c] = uu[(cin0 + r * rstride) * 5 + c];
+    const size_t rstride = (AXIS == 1) ? (size_t)nx : (size_t)nx * ny;  // cells between rows of a
+    const size_t cin0 = (AXIS == 1) ? (((size_t)z * ny + a0) * nx + i0) : (((size_t)a0 * ny + z) * nx + i0);
+    R ru[RW][QU], rb[RW][QB];
+#pragma unroll
+    for (int s = 0; s < RW; s++) {
+        const int r = warp + 8 * s;
+        const R* ur = uu + (cin0 + r * rstride) * 5;
+        const R* br = ub + (cin0 + r * rstride) * 3;
+#pragma unroll
+        for (int q = 0; q < QU; q++)
+            if (r < ta && lane + 32 * q < 5 * ti)
+                ru[s][q] = ur[lane + 32 * q];
+#pragma unroll
+        for (int q = 0; q < QB; q++)
+            if (r < ta && lane + 32 * q < 3 * ti)
+                rb[s][q] = br[lane + 32 * q];
     }
-    for (int e = threadIdx.x; e < ta * ti * 3; e += blockDim.x) {
-        const int r = e / (ti * 3), c = e - r * (ti * 3);
-        sb[r * SB + c] = ub[(cin0 + r * rstride) * 3 + c];
+#pragma unroll
+    for (int s = 0; s < RW; s++) {
+        const int r = warp + 8 * s;
+#pragma unroll
+        for (int q = 0; q < QU; q++)
+            if (r < ta && lane + 32 * q < 5 * ti)
+                su[r * SU + lane + 32 * q] = ru[s][q];
+#pragma unroll
+        for (int q = 0; q < QB; q++)
+            if (r < ta && lane + 32 * q < 3 * ti)
+                sb[r * SB + lane + 32 * q] = rb[s][q];
+    }
+    // output float f of a row is component c of cell aa = f / 5 (f / 3, f / 2)
+    int ou[QU], ob[QB], ow[QW];
+#pragma unroll
+    for (int q = 0; q < QU; q++) {
+        const int f = lane + 32 * q, aa = f / 5;
+        ou[q] = aa * SU + perm_u<AXIS>(f - 5 * aa);
+    }
+#pragma unroll
+    for (int q = 0; q < QB; q++) {
+        const int f = lane + 32 * q, aa = f / 3;
+        ob[q] = aa * SB + perm_b<AXIS>(f - 3 * aa);
+    }
+#pragma unroll
+    for (int q = 0; q < QW; q++) {
+        const int f = lane + 32 * q;
+        ow[q] = (f >> 1) * SU + perm_u<AXIS>(f & 1);
     }
     __syncthreads();
     // output: axis 1 -> dims (ny,nx,nz), cell (a, i, z); axis 2 -> dims (nz,ny,nx), cell (a, z, i)
-    for (int r = 0; r < ti; r++) {
-        const int iv = i0 + r;
-        const size_t cout = (a.axis == 1) ? (((size_t)z * nx + iv) * ny + a0)
-                                          : (((size_t)iv * ny + z) * nz + a0);
-        for (int e = threadIdx.x; e < ta * 5; e += blockDim.x) {
-            const int aa = e / 5, c = e - aa * 5;
-            const int src = (a.axis == 1) ? perm_u<1>(c) : perm_u<2>(c);
-            uo[cout * 5 + e] = su[aa * SU + r * 5 + src];
-        }
-        for (int e = threadIdx.x; e < ta * 3; e += blockDim.x) {
-            const int aa = e / 3, c = e - aa * 3;
-            const int src = (a.axis == 1) ? perm_b<1>(c) : perm_b<2>(c);
-            bo[cout * 3 + e] = sb[aa * SB + r * 3 + src];
-        }
+#pragma unroll
+    for (int s = 0; s < RW; s++) {
+        const int i = warp + 8 * s;
+        if (i >= ti)
+            break;
+        const size_t cout = (AXIS == 1) ? (((size_t)z * nx + i0 + i) * ny + a0) : (((size_t)(i0 + i) * ny + z) * nz + a0);
+#pragma unroll
+        for (int q = 0; q < QU; q++)
+            if (lane + 32 * q < 5 * ta)
+                uo[cout * 5 + lane + 32 * q] = su[ou[q] + 5 * i];
+#pragma unroll
+        for (int q = 0; q < QB; q++)
+            if (lane + 32 * q < 3 * ta)
+                bo[cout * 3 + lane + 32 * q] = sb[ob[q] + 3 * i];
         if (wo) {
-            for (int e = threadIdx.x; e < ta * 2; e += blockDim.x) {
-                const int aa = e / 2, c = e - aa * 2;
-                const int src = (a.axis == 1) ? perm_u<1>(c) : perm_u<2>(c);
-                wo[cout * 2 + e] = su[aa * SU + r * 5 + src];
-            }
+#pragma unroll
+            for (int q = 0; q < QW; q++)
+                if (lane + 32 * q < 2 * ta)
+                    wo[cout * 2 + lane + 32 * q] = su[ow[q] + 5 * i];
         }
     }
 }
 
-template <typename R>
+template <int AXIS, typename R>
 __global__ void __launch_bounds__(256) k_transpose(TransposeArgs a)
 {
     constexpr int kTT = TTile<R>::E;
-    __shared__ R su[kTT * (kTT * 5 + 1)];
-    __shared__ R sb[kTT * (kTT * 3 + 1)];
-    transpose_body<R>(a, su, sb, HwBlock{});
+    __shared__ R su[kTT * (kTT * 5 + 5)];
+    __shared__ R sb[kTT * (kTT * 3 + 3)];
+    const int nbz = (AXIS == 1) ? a.nz : a.ny;  // extent of the untouched axis
+    const int z = blockIdx.z % nbz;
+    select_box(a, blockIdx.z / nbz);
+    transpose_tile<AXIS, R>(a, su, sb, z);
 }
 
 // copy_matrix (C/copy_matrix.c:9-38) as a vectorised device copy.

@@ -68,6 +68,41 @@ int advect_pencils(int nx, int ny);
 
 cudaError_t launch_copy(const void* src, void* dst, size_t bytes, cudaStream_t s);
 
+// Raise a kernel's dynamic shared-memory limit to the device's opt-in maximum
+// minus its static shared memory (once per kernel).  Kernels that stage all
+// their input by TMA ask for the largest shared-memory carveout (they do not
+// use L1 for data), so residency is set by registers and shared memory only.
+template <typename K>
+static cudaError_t allow_smem(K kernel, bool& done, bool tma_staged = false)
+{
+    if (done)
+        return cudaSuccess;
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess)
+        e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess && tma_staged)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    if (e == cudaSuccess)
+        done = true;
+    return e;
+}
+
+// Pencils of any length (mhd_ragged.cuh; FP32): the groups of a pencil of n cells
+// (C = 0: none, see rag_shape), the CFL partials of the fluidx, and the launches.
+struct RagShape {
+    int C, T, G;  // cells per thread, threads and lanes per pencil
+};
+RagShape rag_shape(int n, int ahead);
+int rag_fluidx_parts(int nx, int ny, int nz);
+cudaError_t fluidx_ragged(const FluidxArgs& a, bool exact, cudaStream_t s);
+cudaError_t advect_ragged(const AdvectArgs& a, bool exact, cudaStream_t s);
+
 // Launch-shape knobs set by mhd_tune_set (0 = the planner's own choice).
 enum TuneKey : int {
     TUNE_FLUIDX_THREADS = 0,  // threads per CTA of the register-resident fluidx (64/128/256)

@@ -136,11 +136,15 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, int c0, int c1, i
                  : "memory");
 }
 
-// 4-byte asynchronous global -> shared copy (per thread; completion through
+// 4- and 8-byte asynchronous global -> shared copies (per thread; completion through
 // cp.async groups), used where a tile must be scattered element by element.
 __device__ __forceinline__ void cp_async4(void* dst, const void* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 // 16-byte asynchronous global -> shared copy, not cached in L1 (both
 // addresses 16-byte aligned).
