@@ -438,14 +438,14 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
                     flux[m][s] = lin<R, EX>(R(0.5), lin<R, EX>(R(1), fr[m][s], R(-1), gn), R(0.5),
                                             lin<R, EX>(R(1), dfr, R(-1), dfl));
                 } else {
-                    // branch-free: the reciprocal is taken for every cell.  With a = A/2,
+                    // branch-free: the quotient is taken for every cell.  With a = A/2,
                     // b = B/2: 2ab / (a + b) = AB / (A + B), and every factor dropped is a
-                    // power of two.  The limited differences go straight into the flux,
-                    // which is kept undivided (2 flux; the half goes into the step below).
+                    // power of two.  The flux is kept undivided (2 flux; the half goes into
+                    // the step below).
                     const R pr = dmn * dm[m][s], pl = dln * dl[m][s];
-                    R t = fr[m][s] - gn;
-                    t = fma_if_pos(pr, pr, fast_rcp(dmn + dm[m][s]), t);
-                    flux[m][s] = fma_if_pos(pl, -pl, fast_rcp(dln + dl[m][s]), t);
+                    const R dfr = mul_if_pos(pr, pr, fast_rcp(dmn + dm[m][s]));
+                    const R d = sub_if_pos(pl, dfr, fast_div(pl, dln + dl[m][s]));
+                    flux[m][s] = (fr[m][s] - gn) + d;
                 }
             }
     }

@@ -537,7 +537,12 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
         const int r = it / n, i = it - r * n;
         const int im = (i == 0) ? n - 1 : i - 1;
-        T2[it] = tvdb_prod<R, EX>(VG[it], tvdb_half<R, EX>(BV[it], F1[it], F1[r * n + im], dt));
+        R b1;
+        if constexpr (EX)
+            b1 = tvdb_half<R, EX>(BV[it], F1[it], F1[r * n + im], dt);
+        else
+            b1 = BV[it] - (F1[it] - F1[r * n + im]) * dt * R(0.5);
+        T2[it] = VG[it] * b1;
     }
     __syncthreads();
     // Phase 5: limited upwind flux (C/tvdb.c:54-78).

@@ -39,8 +39,8 @@ __device__ __forceinline__ float rabs<float>(float x)
 // densities are normal, and a limiter quotient is used only where the product
 // of its two differences is positive, so their sum is at least 2^-75.
 // The fluidx and advectbyzx kernels are bound by instruction issue: with
-// these, fma_if_pos and the kept field (mhd_fluidx2.cuh) four 256^3 steps take
-// 9.91 ms plain and 8.60 ms fused, against 10.94 and 9.27 ms before.
+// these, mul_if_pos and the kept field (mhd_fluidx2.cuh) four 256^3 steps take
+// 10.03 ms plain and 8.66 ms fused, against 10.94 and 9.27 ms before, bit for bit.
 template <typename R>
 __device__ __forceinline__ R fast_rcp(R x)
 {
@@ -61,7 +61,7 @@ __device__ __forceinline__ R fast_div(R x, R y)
 template <>
 __device__ __forceinline__ float fast_div<float>(float x, float y)
 {
-    return x * fast_rcp(y);
+    return __fmul_rn(x, fast_rcp(y));
 }
 template <typename R>
 __device__ __forceinline__ R fast_sqrt(R x)
@@ -76,19 +76,27 @@ __device__ __forceinline__ float fast_sqrt<float>(float x)
     return r;
 }
 
-// t + x r where p > 0, else t: one predicated multiply-add (the limited
-// differences are added where they exist; no select and no separate sum).
-__device__ __forceinline__ float fma_if_pos(float p, float x, float r, float t)
+// x r where p > 0, else 0; and t - x where p > 0, else t: predicated, with no
+// select.  (The two limited differences of a flux are rounded one by one, as
+// they always were: a fused multiply-add is faster by 3% of a step, but the
+// closure net amplifies a last-bit change of the state by 1e5.)
+__device__ __forceinline__ float mul_if_pos(float p, float x, float r)
 {
-    asm("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %1, 0f00000000;\n\t@q fma.rn.f32 %0, %2, %3, %0;\n\t}"
-        : "+f"(t)
+    float d = 0.f;
+    asm("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %1, 0f00000000;\n\t@q mul.rn.f32 %0, %2, %3;\n\t}"
+        : "+f"(d)
         : "f"(p), "f"(x), "f"(r));
+    return d;
+}
+__device__ __forceinline__ double mul_if_pos(double p, double x, double r) { return (p > 0.0) ? x * r : 0.0; }
+__device__ __forceinline__ float sub_if_pos(float p, float t, float x)
+{
+    asm("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %1, 0f00000000;\n\t@q sub.rn.f32 %0, %0, %2;\n\t}"
+        : "+f"(t)
+        : "f"(p), "f"(x));
     return t;
 }
-__device__ __forceinline__ double fma_if_pos(double p, double x, double r, double t)
-{
-    return (p > 0.0) ? fma(x, r, t) : t;
-}
+__device__ __forceinline__ double sub_if_pos(double p, double t, double x) { return (p > 0.0) ? t - x : t; }
 
 // ------------------------------------------- EXACT in FP32 without FP64
 //
@@ -458,7 +466,7 @@ __device__ __forceinline__ R tvdb_flux(R vbm, R vb0, R vbp, R vbpp, R vh, R dt)
         const R dp = r_sub(vbp, up ? vb0 : vbpp);
         const R dm = r_sub(vb0, up ? vbm : vbp);
         const R p = r_mul(dm, dp);
-        return r_mul(fma_if_pos(p, p, fast_rcp(r_add(dm, dp)), w), dt);
+        return r_mul(r_add(w, mul_if_pos(p, p, fast_rcp(r_add(dm, dp)))), dt);
     }
 }
 

@@ -1,7 +1,8 @@
 // fluidx and advectbyzx of the x sweep for pencils of any length (FP32): the
 // shapes that the fixed-length register engines (mhd_fluidx2.cuh,
 // mhd_advect2/3/6.cuh) were not laid out for (100, 72, 75, 33 cells), and
-// arrays that are not 16-byte aligned.  Same arithmetic, cell for cell.
+// arrays that are not 16-byte aligned.  Both policies give the bits of the
+// one-thread-per-cell kernels that took these lengths before.
 //
 // A pencil of n cells is held by T = ceil(n / C) threads with C (3, 4 or 5)
 // consecutive cells in registers; the last one holds the remaining L cells and,
@@ -20,8 +21,7 @@
 // issue and latency (the boxes fit in L2).
 //
 // Measured (plain steps, with the transposes of mhd_kernels.cuh): four steps of
-// 100 x 72 x 72 in 1.67 ms before, 1.02 ms now; one step of 200 x 150 x 150 1.27 ms
-// (1.76 ms with the pencils staged piece by piece by all threads).
+// 100 x 72 x 72 in 1.67 ms before, 1.07 ms now; one step of 200 x 150 x 150 1.40 ms.
 #pragma once
 #include "mhd_kernels.cuh"
 #include "mhd_launch.h"
@@ -221,6 +221,29 @@ __device__ __forceinline__ void rag_lds(const float* s, float (&d)[NF])
     }
 }
 
+// cell_flux's FAST form with the roundings that k_fluidx, the kernel of these lengths
+// before, was compiled to (which products went into a multiply-add): the two agree bit for
+// bit, which a run that feeds the state to the closure net needs (the net amplifies a
+// last-bit change by 1e5).
+__device__ __forceinline__ void rag_cell_flux(const float q[5], const float f[3], float v[5], float& ci)
+{
+    constexpr float kG1 = kGammaF - 1.0f, kK = 0.5f * (2.0f - kGammaF);
+    const float ri = fast_rcp(q[0]);
+    const float vx = q[1] * ri;
+    const float mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
+    const float p0 = __fmul_rn(f[0], f[0]);
+    const float bb = __fmaf_rn(f[2], f[2], __fmaf_rn(f[1], f[1], p0));
+    const float ps = __fmaf_rn(kK, bb, __fmul_rn(q[4] - 0.5f * mm * ri, kG1));
+    v[0] = q[1];
+    v[1] = __fsub_rn(__fmaf_rn(q[1], vx, ps), p0);
+    v[2] = q[2] * vx - f[1] * f[0];
+    v[3] = q[3] * vx - f[2] * f[0];
+    const float dot = __fmaf_rn(f[2], q[3], __fmaf_rn(f[0], q[1], __fmul_rn(f[1], q[2])));
+    v[4] = __fmaf_rn(__fadd_rn(q[4], ps), vx, -__fmul_rn(__fmul_rn(f[0], dot), ri));
+    const float p = ps - 0.5f * bb;
+    ci = fabsf(vx) + fast_sqrt(fabsf((bb + kGammaF * p) * ri));
+}
+
 // C/fluidx.c:19-102, C/tvd1.c:8-118, C/mhdflux.c:9-72; see fluidx2_body for the
 // arithmetic, which this repeats expression by expression.
 template <bool EX, int C, int D>
@@ -292,42 +315,34 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
 #pragma unroll
         for (int m = 0; m < C; m++) {
             const R b0n = (m + 1 < C) ? bj[3 * (m + 1)] : b1next;
-            if constexpr (EX) {
-                f[m][0] = R(0.5) * bj[3 * m] + R(0.5) * b0n;
-                f[m][1] = R(0.5) * bj[3 * m + 1] + bp[3 * m + 1] / R(2);
-                f[m][2] = R(0.5) * bj[3 * m + 2] + bk[3 * m + 2] / R(2);
-            } else {
-                f[m][0] = R(0.5) * (bj[3 * m] + b0n);
-                f[m][1] = R(0.5) * (bj[3 * m + 1] + bp[3 * m + 1]);
-                f[m][2] = R(0.5) * (bj[3 * m + 2] + bk[3 * m + 2]);
-            }
+            f[m][0] = R(0.5) * bj[3 * m] + R(0.5) * b0n;
+            f[m][1] = R(0.5) * bj[3 * m + 1] + bp[3 * m + 1] / R(2);
+            f[m][2] = R(0.5) * bj[3 * m + 2] + bk[3 * m + 2] / R(2);
         }
     }
 
-    // fluxes of the state w: fr = c w + v, gl = c w - v (C/tvd1.c:33-49, 51-69)
+    // fluxes of the state w: fr = c (w + v / c), gl = c (w - v / c) (C/tvd1.c:33-49, 51-69).
+    // (FAST: the expressions of k_fluidx, which the compiler contracts alike)
     R fr[C][5], gl[C][5];
     auto fluxes = [&](const R (&w)[C][5], R* rd) {
         R v[C][5], cm = R(0);
 #pragma unroll
         for (int m = 0; m < C; m++) {
             R ci;
-            cell_flux<R, EX>(w[m], f[m], v[m], ci);
+            if constexpr (EX)
+                cell_flux<R, EX>(w[m], f[m], v[m], ci);
+            else
+                rag_cell_flux(w[m], f[m], v[m], ci);
             cm = fmaxf(cm, ci);
         }
         const R c = g.max(cm, rd);
 #pragma unroll
         for (int m = 0; m < C; m++) {
-            if constexpr (EX)
-                scale_flux<R, EX>(v[m], c);
+            scale_flux<R, EX>(v[m], c);
 #pragma unroll
             for (int s = 0; s < 5; s++) {
-                if constexpr (EX) {
-                    fr[m][s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[m][s], R(1), v[m][s]));
-                    gl[m][s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[m][s], R(-1), v[m][s]));
-                } else {
-                    fr[m][s] = fmaf(c, w[m][s], v[m][s]);
-                    gl[m][s] = fmaf(c, w[m][s], -v[m][s]);
-                }
+                fr[m][s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[m][s], R(1), v[m][s]));
+                gl[m][s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[m][s], R(-1), v[m][s]));
             }
         }
     };
@@ -344,7 +359,7 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
                                      lin<R, EX>(R(1), flux[m][s], R(-1), (m > 0) ? flux[m - 1][s] : fp[s]));
     };
 
-    // ---- stage 1 (FAST keeps its fluxes undivided, the half is in the step)
+    // ---- stage 1
     fluxes(q, red);
     {
         R gn[1][5];
@@ -354,9 +369,9 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
 #pragma unroll
             for (int s = 0; s < 5; s++) {
                 const R x = (m + 1 < C) ? gl[m + 1][s] : gn[0][s];
-                flux[m][s] = EX ? lin<R, EX>(R(0.5), fr[m][s], R(-0.5), x) : fr[m][s] - x;
+                flux[m][s] = lin<R, EX>(R(0.5), fr[m][s], R(-0.5), x);
             }
-        update(q, EX ? R(-0.5) * dt : R(-0.25) * dt);
+        update(q, R(-0.5) * dt);
     }
     // ---- stage 2
     fluxes(q, red + 16);
@@ -369,8 +384,8 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
 #pragma unroll
             for (int s = 0; s < 5; s++) {
                 const R p = (m > 0) ? fr[m - 1][s] : frp[s], x = (m + 1 < C) ? gl[m + 1][s] : gn[0][s];
-                d[m][s] = EX ? lin<R, EX>(R(0.5), fr[m][s], R(-0.5), p) : fr[m][s] - p;
-                d[m][5 + s] = EX ? lin<R, EX>(R(0.5), gl[m][s], R(-0.5), x) : gl[m][s] - x;
+                d[m][s] = lin<R, EX>(R(0.5), fr[m][s], R(-0.5), p);
+                d[m][5 + s] = lin<R, EX>(R(0.5), gl[m][s], R(-0.5), x);
             }
         g.template next<10, 1>(d, dn, seam, 0);
 #pragma unroll
@@ -379,18 +394,12 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
             for (int s = 0; s < 5; s++) {
                 const R dr = (m + 1 < C) ? d[m + 1][s] : dn[0][s], dl = (m + 1 < C) ? d[m + 1][5 + s] : dn[0][5 + s];
                 const R x = (m + 1 < C) ? gl[m + 1][s] : gn[0][s];
-                if constexpr (EX) {
-                    const R a1 = vanleer<R, EX>(dr, d[m][s]), a2 = vanleer<R, EX>(dl, d[m][5 + s]);
-                    flux[m][s] = lin<R, EX>(R(0.5), lin<R, EX>(R(1), fr[m][s], R(-1), x), R(0.5),
-                                            lin<R, EX>(R(1), a1, R(-1), a2));
-                } else {
-                    const R pr = dr * d[m][s], pl = dl * d[m][5 + s];
-                    const R t = fma_if_pos(pr, pr, fast_rcp(dr + d[m][s]), fr[m][s] - x);
-                    flux[m][s] = fma_if_pos(pl, -pl, fast_rcp(dl + d[m][5 + s]), t);
-                }
+                const R a1 = vanleer<R, EX>(dr, d[m][s]), a2 = vanleer<R, EX>(dl, d[m][5 + s]);
+                flux[m][s] = lin<R, EX>(R(0.5), lin<R, EX>(R(1), fr[m][s], R(-1), x), R(0.5),
+                                        lin<R, EX>(R(1), a1, R(-1), a2));
             }
         load_q(q);
-        update(q, EX ? -dt : R(-0.5) * dt);
+        update(q, -dt);
     }
 #pragma unroll
     for (int m = 0; m < C; m++)
@@ -468,6 +477,13 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
     }
 }
 
+// Half step of tvdb, in both policies with the reference's roundings: the product, then
+// b - x / 2 once (FAST: the bits of k_advect, the kernel of these lengths before).
+__device__ __forceinline__ float rag_half(float bv, float f1, float fm, float dt)
+{
+    return __fmaf_rn(-0.5f, __fmul_rn(__fsub_rn(f1, fm), dt), bv);
+}
+
 // One tvdb row of a group, as tvdb_row (mhd_advect2.cuh) for these groups.
 template <bool EX, int C, int D>
 __device__ __forceinline__ void rag_tvdb_row(const RagGroup<C, D>& g, const float (&vr)[C][1], const float (&bv)[C],
@@ -497,7 +513,7 @@ __device__ __forceinline__ void rag_tvdb_row(const RagGroup<C, D>& g, const floa
         float vb[C];
 #pragma unroll
         for (int m = 0; m < C; m++)
-            vb[m] = tvdb_prod<float, EX>(t[m][0], tvdb_half<float, EX>(bv[m], x[m][0], m > 0 ? x[m - 1][0] : l[0], dt));
+            vb[m] = tvdb_prod<float, EX>(t[m][0], rag_half(bv[m], x[m][0], m > 0 ? x[m - 1][0] : l[0], dt));
 #pragma unroll
         for (int m = 0; m < C; m++)
             x[m][0] = vb[m];
@@ -529,7 +545,7 @@ __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, i
 {
     select_box(a, blockIdx.z);
     extern __shared__ __align__(16) float rag_smem[];
-    const int n = a.nx, ny = a.ny, nz = a.nz, J = a.P, tid = threadIdx.x, nt = blockDim.x, tc = sh.T * C;
+    const int n = a.nx, ny = a.ny, nz = a.nz, J = a.P, tid = threadIdx.x, tc = sh.T * C;
     const RagGroup<C, D> g(sh, tid);
     const int j0 = blockIdx.x * J, k0 = blockIdx.y * a.K, k1 = min(k0 + a.K, nz);
     const int np = min(J, ny - j0), w = min(tid / sh.G, np);  // the group's pencil; np: the halo pencil
@@ -585,7 +601,7 @@ __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, i
                     float (&v)[C][1]) {
 #pragma unroll
         for (int m = 0; m < C; m++)
-            v[m][0] = tvdb_face<float, EX>(ml[m], mc[m], rl[m], rc[m]);
+            v[m][0] = __fdiv_rn(__fadd_rn(ml[m], mc[m]), __fadd_rn(rl[m], rc[m]));
     };
 
     if (pb == 16 && tid == 0) {
