@@ -376,7 +376,7 @@ __device__ __forceinline__ void tc_epilogue_row(const uint32_t (&r)[32], size_t 
 template <int COUT, int EPI>
 __device__ __forceinline__ void tc_epilogue_row_tab(const uint32_t (&r)[32], size_t v, const float* __restrict__ bias,
                                                     void* __restrict__ y, bf16* __restrict__ zsave,
-                                                    const bf16* __restrict__ zprev,
+                                                    const uint4 (&zp)[COUT / 8],
                                                     const unsigned short* __restrict__ gelu_tab,
                                                     const float* __restrict__ grad_tab)
 {
@@ -393,7 +393,8 @@ __device__ __forceinline__ void tc_epilogue_row_tab(const uint32_t (&r)[32], siz
                                ((uint32_t)__ldg(gelu_tab + (bits >> 16)) << 16);
             *reinterpret_cast<uint32_t*>(o1 + c) = g;
         } else {
-            const uint32_t zb = *reinterpret_cast<const uint32_t*>(zprev + v * COUT + c);
+            const uint4 z4 = zp[c / 8];
+            const uint32_t zb = (c & 4) ? ((c & 2) ? z4.w : z4.z) : ((c & 2) ? z4.y : z4.x);
             *reinterpret_cast<__nv_bfloat162*>(o1 + c) =
                 __floats2bfloat162_rn(v0 * __ldg(grad_tab + (zb & 0xFFFFu)), v1 * __ldg(grad_tab + (zb >> 16)));
         }
@@ -699,6 +700,23 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
         const int q = warp & 3;
         for (long long i = 0; i < mine; i++) {
             const int st = (int)(i % NT);
+            int box, z0, y0, x0;
+            coords((long long)blockIdx.x + i * gridDim.x, box, z0, y0, x0);
+            const int m = q * 32 + lane, vx = m >> 3, vy = m & 7;
+            const size_t v = (((size_t)box * n + z0) * n + (y0 + vy)) * n + (x0 + vx);
+            // the previous layer's pre-activations of both rows, in 16-byte pieces, while the
+            // tile's MMAs run (read pair by pair after them, they made this kind take 140 us
+            // at 4 boxes of 64^3 where the forward kind takes 52)
+            uint4 zp0[COUT / 8], zp1[COUT / 8];
+            if constexpr (EPI == EPI_DGRAD) {
+                const uint4* s0 = reinterpret_cast<const uint4*>(zprev + v * COUT);
+                const uint4* s1 = reinterpret_cast<const uint4*>(zprev + (v + (size_t)n * n) * COUT);
+#pragma unroll
+                for (int c = 0; c < COUT / 8; c++) {
+                    zp0[c] = __ldg(s0 + c);
+                    zp1[c] = __ldg(s1 + c);
+                }
+            }
             if (!mhd::mbar_wait_bounded(&t_full[st], (uint32_t)((i / NT) & 1), err))
                 break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -709,12 +727,8 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
             __syncwarp();
             if (lane == 0)
                 mbar_arrive1(&t_empty[st]);
-            int box, z0, y0, x0;
-            coords((long long)blockIdx.x + i * gridDim.x, box, z0, y0, x0);
-            const int m = q * 32 + lane, vx = m >> 3, vy = m & 7;
-            const size_t v = (((size_t)box * n + z0) * n + (y0 + vy)) * n + (x0 + vx);
-            tc_epilogue_row_tab<COUT, EPI>(r0, v, bias, y, zsave, zprev, gelu_tab, grad_tab);
-            tc_epilogue_row_tab<COUT, EPI>(r1, v + (size_t)n * n, bias, y, zsave, zprev, gelu_tab, grad_tab);
+            tc_epilogue_row_tab<COUT, EPI>(r0, v, bias, y, zsave, zp0, gelu_tab, grad_tab);
+            tc_epilogue_row_tab<COUT, EPI>(r1, v + (size_t)n * n, bias, y, zsave, zp1, gelu_tab, grad_tab);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -724,8 +738,13 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
 }
 
 // dW(co, tap, ci) = sum_v dz(v, co) a(v + off(tap), ci).  Warp w owns the taps
-// t == w mod WT and the k-steps (16 voxels) s == w / WT mod WK.  Each warp
-// writes its FP32 partial sums to part[cta][w / WT][tap][co][ci].
+// t == w mod WT and the k-steps (16 voxels) s == w / WT mod WK.  The tiles are
+// dealt over `nsets` sets; each warp writes its FP32 partial sums of a set to
+// part[set][w / WT][tap][co][ci], so a sum's length and order depend on the sets
+// only.  A CTA works its sets off one after the other with two tile buffers: the
+// next tile's copies are in flight while the current one is multiplied.  The 150
+// registers of the 3^3 kind let one CTA of nine warps on an SM, so without that
+// every tile waited for its own copies (4 boxes of 64^3: 214 us before).
 template <int CIN, int COUTP, int KS>
 struct WgradShape {
     static constexpr int TAPS = KS * KS * KS;
@@ -738,15 +757,14 @@ struct WgradShape {
 template <int CIN, int COUTP, int KS>
 __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
     k_wgrad(const bf16* __restrict__ a, const bf16* __restrict__ dz, float* __restrict__ part, int n,
-            long long ntiles)
+            long long ntiles, int nsets)
 {
     using S = WgradShape<CIN, COUTP, KS>;
     using HL = Halo<KS>;
     constexpr int RS = row_bytes(CIN), RZ = row_bytes(COUTP);
     constexpr int MTL = COUTP / 16, NTL = CIN / 8;
     extern __shared__ __align__(16) unsigned char sm[];
-    unsigned char* sa = sm;                               // [ROWS][RS]
-    unsigned char* sz = sm + (size_t)HL::ROWS * RS;       // [TV][RZ]
+    constexpr size_t kBuf = (size_t)HL::ROWS * RS + (size_t)TV * RZ;  // halo rows of a, rows of dz
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wt = warp % S::WT, wk = warp / S::WT;
@@ -765,22 +783,38 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
                 for (int q = 0; q < 4; q++)
                     acc[p][i][j][q] = 0.f;
 
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    auto load = [&](long long tile, int buf) {
         const TileIdx t = tile_of(tile, n);
-        __syncthreads();
+        unsigned char* sa = sm + buf * kBuf;
+        unsigned char* sz = sa + (size_t)HL::ROWS * RS;
         load_rows<CIN, KS>(sa, a, t, n);
-        {
-            constexpr int CH = COUTP * 2 / 16;
-            const size_t box0 = (size_t)t.box * n * n * n;
-            for (int e = threadIdx.x; e < TV * CH; e += blockDim.x) {
-                const int row = e / CH, ch = e - row * CH;
-                const int tx = row % TX, ty = (row / TX) % TY, tz = row / (TX * TY);
-                const bf16* s = dz + (box0 + ((size_t)(t.z0 + tz) * n + (t.y0 + ty)) * n + (t.x0 + tx)) * COUTP + ch * 8;
-                cp_async16(sz + (size_t)row * RZ + ch * 16, s);
-            }
+        constexpr int CH = COUTP * 2 / 16;
+        const size_t box0 = (size_t)t.box * n * n * n;
+        for (int e = threadIdx.x; e < TV * CH; e += blockDim.x) {
+            const int row = e / CH, ch = e - row * CH;
+            const int tx = row % TX, ty = (row / TX) % TY, tz = row / (TX * TY);
+            const bf16* s = dz + (box0 + ((size_t)(t.z0 + tz) * n + (t.y0 + ty)) * n + (t.x0 + tx)) * COUTP + ch * 8;
+            cp_async16(sz + (size_t)row * RZ + ch * 16, s);
         }
-        cp_async_wait_all();
+    };
+    int set = blockIdx.x, buf = 0;
+    long long tile = set;
+    load(tile, 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    while (set < nsets) {
+        int nset = set;
+        long long ntile = tile + nsets;
+        if (ntile >= ntiles) {
+            nset += gridDim.x;
+            ntile = nset;
+        }
+        if (nset < nsets)
+            load(ntile, buf ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
+        const unsigned char* sa = sm + buf * kBuf;
+        const unsigned char* sz = sa + (size_t)HL::ROWS * RS;
 
 #pragma unroll 1
         for (int s = wk; s < TV / 16; s += S::WK) {
@@ -810,25 +844,31 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
                 }
             }
         }
-    }
-    // partials: part[cta][wk][tap][co][ci]
-    float* base = part + ((size_t)blockIdx.x * S::WK + wk) * S::TAPS * COUTP * CIN;
+        if (nset != set) {  // the set's last tile: its partials
+            float* base = part + ((size_t)set * S::WK + wk) * S::TAPS * COUTP * CIN;
 #pragma unroll
-    for (int p = 0; p < S::TPW; p++) {
-        const int tap = wt + p * S::WT;
-        if (tap >= S::TAPS)
-            break;
+            for (int p = 0; p < S::TPW; p++) {
+                const int tap = wt + p * S::WT;
+                if (tap >= S::TAPS)
+                    break;
 #pragma unroll
-        for (int i = 0; i < MTL; i++)
+                for (int i = 0; i < MTL; i++)
 #pragma unroll
-            for (int j = 0; j < NTL; j++)
+                    for (int j = 0; j < NTL; j++)
 #pragma unroll
-                for (int hr = 0; hr < 2; hr++) {
-                    const int co = i * 16 + (lane >> 2) + 8 * hr, ci = j * 8 + 2 * (lane & 3);
-                    float* d = base + ((size_t)tap * COUTP + co) * CIN + ci;
-                    d[0] = acc[p][i][j][2 * hr];
-                    d[1] = acc[p][i][j][2 * hr + 1];
-                }
+                        for (int hr = 0; hr < 2; hr++) {
+                            const int co = i * 16 + (lane >> 2) + 8 * hr, ci = j * 8 + 2 * (lane & 3);
+                            float* d = base + ((size_t)tap * COUTP + co) * CIN + ci;
+                            d[0] = acc[p][i][j][2 * hr];
+                            d[1] = acc[p][i][j][2 * hr + 1];
+                            acc[p][i][j][2 * hr] = acc[p][i][j][2 * hr + 1] = 0.f;
+                        }
+            }
+        }
+        __syncthreads();  // the buffer is read
+        buf ^= 1;
+        set = nset;
+        tile = ntile;
     }
 }
 
@@ -1159,6 +1199,30 @@ __global__ void k_diff(const float* __restrict__ ua, const float* __restrict__ b
 // round-off: a run already at its final time).  dt may be absent (always correct).
 __device__ __forceinline__ bool skip_step(const float* dt, float dt_min) { return dt && !(*dt > dt_min); }
 
+// dst[c] += the block's sum of s[c] (256 threads): one atomic per block and sum.  All
+// atomics of a launch hit the same few words, one after the other: with one per warp and
+// eight blocks per SM they were nearly all of k_apply0's 56 us at 64^3.
+template <int N>
+__device__ __forceinline__ void block_add(const double (&s)[N], double* dst)
+{
+    __shared__ double red[8][N];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+        const double t = mhd_warp_sum_d(s[c]);
+        if (lane == 0)
+            red[w][c] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            t += red[k][threadIdx.x];
+        atomicAdd(dst + threadIdx.x, t);
+    }
+}
+
 // esum[2 + c] += sum over the box of out[.][c], c < 5 (the fluid corrections' means are removed,
 // so the correction conserves mass, momentum and energy as the filtered fine step does)
 __global__ void k_apply0(const float* __restrict__ out, size_t nv, double* __restrict__ esum,
@@ -1171,12 +1235,7 @@ __global__ void k_apply0(const float* __restrict__ out, size_t nv, double* __res
 #pragma unroll
         for (int c = 0; c < 5; c++)
             s[c] += out[v * 8 + c];
-#pragma unroll
-    for (int c = 0; c < 5; c++) {
-        const double t = mhd_warp_sum_d(s[c]);
-        if ((threadIdx.x & 31) == 0)
-            atomicAdd(&esum[2 + c], t);
-    }
+    block_add<5>(s, esum + 2);
 }
 
 // candidate = state + alpha * correction (fluid part with its box mean removed) into (ut, bt);
@@ -1211,12 +1270,8 @@ __global__ void k_apply1(const float* __restrict__ u, const float* __restrict__ 
         e0 += u[v * 5 + 4];
         e1 += ut[v * 5 + 4];
     }
-    e0 = mhd_warp_sum_d(e0);
-    e1 = mhd_warp_sum_d(e1);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&esum[0], e0);
-        atomicAdd(&esum[1], e1);
-    }
+    const double e[2] = {e0, e1};
+    block_add<2>(e, esum);
 }
 
 // positivity of the candidate (it needs the neighbours' candidate faces: a second pass)
@@ -1421,8 +1476,8 @@ size_t wgrad_parts(int nb, int n)
 {
     using S = WgradShape<CIN, COUTP, KS>;
     const long long ntiles = (long long)nb * (n / TX) * (n / TY) * (n / TZ);
-    const long long grid = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
-    return (size_t)grid * S::WK;
+    const long long nsets = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
+    return (size_t)nsets * S::WK;
 }
 
 template <int CIN, int COUTP, int KS>
@@ -1431,7 +1486,7 @@ int launch_wgrad(const void* a, const void* dz, float* part, float* dw, int cor,
 {
     using S = WgradShape<CIN, COUTP, KS>;
     using HL = Halo<KS>;
-    const size_t smem = (size_t)HL::ROWS * row_bytes(CIN) + (size_t)TV * row_bytes(COUTP);
+    const size_t smem = 2 * ((size_t)HL::ROWS * row_bytes(CIN) + (size_t)TV * row_bytes(COUTP));
     static bool attr = false;
     if (!attr) {
         if (set_smem(k_wgrad<CIN, COUTP, KS>, smem) != cudaSuccess)
@@ -1439,13 +1494,15 @@ int launch_wgrad(const void* a, const void* dz, float* part, float* dw, int cor,
         attr = true;
     }
     const long long ntiles = (long long)nb * (n / TX) * (n / TY) * (n / TZ);
-    const long long grid = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
-    k_wgrad<CIN, COUTP, KS><<<(unsigned)grid, S::THREADS, smem, s>>>(static_cast<const bf16*>(a),
-                                                                      static_cast<const bf16*>(dz), part, n, ntiles);
+    const long long nsets = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
+    const long long resident = (long long)sms() * (KS == 1 ? 2 : 1);  // CTAs an SM holds: by registers, by shared memory
+    const long long grid = nsets < resident ? nsets : resident;
+    k_wgrad<CIN, COUTP, KS><<<(unsigned)grid, S::THREADS, smem, s>>>(
+        static_cast<const bf16*>(a), static_cast<const bf16*>(dz), part, n, ntiles, (int)nsets);
     if (cudaGetLastError() != cudaSuccess)
         return MHD_ERR_CUDA;
     const size_t len = (size_t)cor * S::TAPS * cir;
-    k_wsum<<<(unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s>>>(part, (int)(grid * S::WK), S::TAPS, COUTP, CIN,
+    k_wsum<<<(unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s>>>(part, (int)(nsets * S::WK), S::TAPS, COUTP, CIN,
                                                                     cor, cir, dw);
     return st(cudaGetLastError());
 }
@@ -1654,11 +1711,12 @@ extern "C" MHD_API int mhd_cl_apply(float* u, float* b, const float* out, int n,
         cudaMemsetAsync(esum, 0, 8 * sizeof(double), s) != cudaSuccess)
         return MHD_ERR_CUDA;
     const unsigned blocks = blocks_for(nv, 256);
-    k_apply0<<<blocks, 256, 0, s>>>(out, nv, esum, dt, dt_min);
+    const unsigned rblocks = blocks < 2u * (unsigned)sms() ? blocks : 2u * (unsigned)sms();  // of the reductions
+    k_apply0<<<rblocks, 256, 0, s>>>(out, nv, esum, dt, dt_min);
     for (int a = 0; a < 3; a++) {  // the full correction, else half, else a quarter, else none
         if (a)
             k_apply_next<<<1, 1, 0, s>>>(flags, esum);
-        k_apply1<<<blocks, 256, 0, s>>>(u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp, esum, flags, dt,
+        k_apply1<<<rblocks, 256, 0, s>>>(u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp, esum, flags, dt,
                                         dt_min);
         k_apply2<<<blocks, 256, 0, s>>>(u_tmp, b_tmp, n, flags, dt, dt_min);
         k_apply3<<<blocks, 256, 0, s>>>(u, b, u_tmp, b_tmp, nv, flags, esum, ecap, fallbacks, a == 2, dt, dt_min);
