@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(128) k_conv(const bf16* __restrict__ x, const 
                                               bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n,
                                               long long ntiles)
 {
+    mhd::after_previous();
     using HL = Halo<KS>;
     constexpr int TAPS = KS * KS * KS;
     constexpr int RS = row_bytes(CIN);
@@ -443,6 +444,7 @@ __global__ void __launch_bounds__(256, 1) k_conv_tc(const bf16* __restrict__ x, 
                                                      bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n,
                                                      long long ntiles, int* err)
 {
+    mhd::after_previous();
     static_assert(COUT == 32, "one tile's accumulators are 2 x 32 TMEM columns");
     constexpr int CH = CIN / 8;
     constexpr int KC = 27 * CH;                  // K chunks of the weights
@@ -598,6 +600,7 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
                void* __restrict__ y, bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n, long long ntiles,
                int* err, const unsigned short* __restrict__ gelu_tab, const float* __restrict__ grad_tab)
 {
+    mhd::after_previous();
     static_assert(COUT == 32, "one tile's accumulators are 2 x 32 TMEM columns");
     constexpr int CH = CIN / 8, NA = tc2_stages<CIN>(), NT = kTc2NT;
     constexpr int KC = 27 * CH;                  // K chunks of the weights
@@ -705,8 +708,7 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
             const int m = q * 32 + lane, vx = m >> 3, vy = m & 7;
             const size_t v = (((size_t)box * n + z0) * n + (y0 + vy)) * n + (x0 + vx);
             // the previous layer's pre-activations of both rows, in 16-byte pieces, while the
-            // tile's MMAs run (read pair by pair after them, they made this kind take 140 us
-            // at 4 boxes of 64^3 where the forward kind takes 52)
+            // tile's MMAs run
             uint4 zp0[COUT / 8], zp1[COUT / 8];
             if constexpr (EPI == EPI_DGRAD) {
                 const uint4* s0 = reinterpret_cast<const uint4*>(zprev + v * COUT);
@@ -759,6 +761,7 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
     k_wgrad(const bf16* __restrict__ a, const bf16* __restrict__ dz, float* __restrict__ part, int n,
             long long ntiles, int nsets)
 {
+    mhd::after_previous();
     using S = WgradShape<CIN, COUTP, KS>;
     using HL = Halo<KS>;
     constexpr int RS = row_bytes(CIN), RZ = row_bytes(COUTP);
@@ -882,6 +885,7 @@ constexpr int kSumWarps = 8;
 __global__ void __launch_bounds__(kSumWarps * 32) k_sum_parts(const float* __restrict__ part, int nparts,
                                                              size_t stride, size_t len, float* __restrict__ out)
 {
+    mhd::after_previous();
     __shared__ float red[kSumWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const size_t e = (size_t)blockIdx.x * 32 + lane;
@@ -907,6 +911,7 @@ constexpr int kWsumWarps = kSumWarps;
 __global__ void __launch_bounds__(kWsumWarps * 32) k_wsum(const float* __restrict__ part, int nparts, int taps,
                                                          int cop, int cip, int cor, int cir, float* __restrict__ dw)
 {
+    mhd::after_previous();
     __shared__ float red[kWsumWarps][32];
     const size_t len = (size_t)cor * taps * cir, stride = (size_t)taps * cop * cip;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -943,6 +948,7 @@ __global__ void __launch_bounds__(kWsumWarps * 32) k_wsum(const float* __restric
 __global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ x, int C, size_t count,
                                                 float* __restrict__ part)
 {
+    mhd::after_previous();
     __shared__ float red[8][32];
     const int Q = C / 8;  // 16-byte chunks per row
     const int q = threadIdx.x % Q, rows = blockDim.x / Q, r0 = threadIdx.x / Q;
@@ -1000,6 +1006,7 @@ __device__ __forceinline__ size_t vidx(int box, int k, int j, int i, int n)
 __global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ tgt, bf16* __restrict__ dout,
                         float* __restrict__ rb_out, float* __restrict__ lpart, int nb, int n, float gscale)
 {
+    mhd::after_previous();
     __shared__ float red[32];
     const size_t nv = (size_t)nb * n * n * n;
     float ls = 0.f;
@@ -1054,6 +1061,7 @@ __global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ 
 // dout[5..7] = gscale * curl^T(rb)
 __global__ void k_loss2(const float* __restrict__ rb, bf16* __restrict__ dout, int nb, int n, float gscale)
 {
+    mhd::after_previous();
     const size_t nv = (size_t)nb * n * n * n;
     for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)((v / ((size_t)n * n)) % n);
@@ -1080,6 +1088,7 @@ __global__ void k_features(const float* __restrict__ u, const float* __restrict_
                            const float* __restrict__ mean, const float* __restrict__ inv_std,
                            float* __restrict__ raw, bf16* __restrict__ xo)
 {
+    mhd::after_previous();
     const size_t nv = (size_t)n * n * n;
     for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)(v / ((size_t)n * n));
@@ -1228,6 +1237,7 @@ __device__ __forceinline__ void block_add(const double (&s)[N], double* dst)
 __global__ void k_apply0(const float* __restrict__ out, size_t nv, double* __restrict__ esum,
                          const float* __restrict__ dt, float dt_min)
 {
+    mhd::after_previous();
     if (skip_step(dt, dt_min))
         return;
     double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -1246,6 +1256,7 @@ __global__ void k_apply1(const float* __restrict__ u, const float* __restrict__ 
                          float* __restrict__ bt, double* __restrict__ esum, const int* __restrict__ flags,
                          const float* __restrict__ dt, float dt_min)
 {
+    mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
         return;
     const size_t nv = (size_t)n * n * n;
@@ -1278,6 +1289,7 @@ __global__ void k_apply1(const float* __restrict__ u, const float* __restrict__ 
 __global__ void k_apply2(const float* __restrict__ ut, const float* __restrict__ bt, int n, int* __restrict__ flags,
                          const float* __restrict__ dt, float dt_min)
 {
+    mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
         return;
     const size_t nv = (size_t)n * n * n;
@@ -1304,6 +1316,7 @@ __global__ void k_apply3(float* __restrict__ u, float* __restrict__ b, const flo
                          const double* __restrict__ esum, float ecap, long long* __restrict__ fallbacks, int last,
                          const float* __restrict__ dt, float dt_min)
 {
+    mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
         return;
     const bool energy_ok = fabs(esum[1] - esum[0]) <= (double)ecap * fabs(esum[0]);
@@ -1326,6 +1339,7 @@ __global__ void k_adamw(float* __restrict__ p, const float* __restrict__ g, floa
                         float* __restrict__ v, size_t count, float lr, float b1, float b2, float eps, float wd,
                         float c1, float c2)
 {
+    mhd::after_previous();
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x) {
         const float gg = g[e];
         const float mm = b1 * m[e] + (1.f - b1) * gg;
@@ -1342,6 +1356,7 @@ __global__ void k_adamw(float* __restrict__ p, const float* __restrict__ g, floa
 __global__ void k_pack(const float* __restrict__ w, int cor, int cir, int taps, int cop, int cip,
                        bf16* __restrict__ wf, bf16* __restrict__ wd)
 {
+    mhd::after_previous();
     const size_t tot = (size_t)cop * taps * cip;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
         const int ci = (int)(e % cip), tap = (int)((e / cip) % taps), co = (int)(e / ((size_t)cip * taps));
@@ -1392,9 +1407,8 @@ int launch_conv(const void* x, const void* w, const float* bias, void* y, void* 
     const long long ntiles = (long long)nb * (n / TX) * (n / TY) * (n / TZ);
     const int per_sm = smem > 110 * 1024 ? 1 : 2;
     const long long grid = ntiles < (long long)sms() * per_sm * 2 ? ntiles : (long long)sms() * per_sm * 2;
-    k_conv<CIN, COUT, KS, EPI><<<(unsigned)grid, 128, smem, s>>>(
-        static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave),
-        static_cast<const bf16*>(zprev), n, ntiles);
+    mhd::launch_after(k_conv<CIN, COUT, KS, EPI>, (unsigned)grid, 128, smem, s, static_cast<const bf16*>(x),
+        static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave), static_cast<const bf16*>(zprev), n, ntiles);
     return st(cudaGetLastError());
 }
 
@@ -1434,7 +1448,7 @@ int launch_conv_tc2(const void* x, const void* w, const float* bias, void* y, vo
     }
     const long long ntiles = (long long)nb * (n / TCX) * (n / TCY) * (n / TCZ);
     const long long grid = ntiles < (long long)sms() ? ntiles : (long long)sms();
-    k_conv_tc2<CIN, COUT, EPI><<<(unsigned)grid, kTc2Warps * 32, smem, s>>>(
+    mhd::launch_after(k_conv_tc2<CIN, COUT, EPI>, (unsigned)grid, kTc2Warps * 32, smem, s,
         static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave),
         static_cast<const bf16*>(zprev), n, ntiles, g_tc_err, g_gelu_tab, g_grad_tab);
     return st(cudaGetLastError());
@@ -1463,9 +1477,9 @@ int launch_conv_tc(const void* x, const void* w, const float* bias, void* y, voi
         return MHD_ERR_NOMEM;
     const long long ntiles = (long long)nb * (n / TCX) * (n / TCY) * (n / TCZ);
     const long long grid = ntiles < (long long)sms() ? ntiles : (long long)sms();
-    k_conv_tc<CIN, COUT, EPI><<<(unsigned)grid, 256, smem, s>>>(
-        static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave),
-        static_cast<const bf16*>(zprev), n, ntiles, g_tc_err);
+    mhd::launch_after(k_conv_tc<CIN, COUT, EPI>, (unsigned)grid, 256, smem, s, static_cast<const bf16*>(x),
+        static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave), static_cast<const bf16*>(zprev), n,
+        ntiles, g_tc_err);
     return st(cudaGetLastError());
 }
 
@@ -1497,13 +1511,13 @@ int launch_wgrad(const void* a, const void* dz, float* part, float* dw, int cor,
     const long long nsets = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
     const long long resident = (long long)sms() * (KS == 1 ? 2 : 1);  // CTAs an SM holds: by registers, by shared memory
     const long long grid = nsets < resident ? nsets : resident;
-    k_wgrad<CIN, COUTP, KS><<<(unsigned)grid, S::THREADS, smem, s>>>(
-        static_cast<const bf16*>(a), static_cast<const bf16*>(dz), part, n, ntiles, (int)nsets);
+    mhd::launch_after(k_wgrad<CIN, COUTP, KS>, (unsigned)grid, S::THREADS, smem, s, static_cast<const bf16*>(a),
+        static_cast<const bf16*>(dz), part, n, ntiles, (int)nsets);
     if (cudaGetLastError() != cudaSuccess)
         return MHD_ERR_CUDA;
     const size_t len = (size_t)cor * S::TAPS * cir;
-    k_wsum<<<(unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s>>>(part, (int)(nsets * S::WK), S::TAPS, COUTP, CIN,
-                                                                    cor, cir, dw);
+    mhd::launch_after(k_wsum, (unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s, part, (int)(nsets * S::WK),
+        S::TAPS, COUTP, CIN, cor, cir, dw);
     return st(cudaGetLastError());
 }
 
@@ -1608,11 +1622,11 @@ extern "C" MHD_API int mhd_cl_colsum(const void* x, int channels, long long coun
     const int threads = 256, blocks = 256;  // blocks: the scratch holds 256 * channels partials
     if (reinterpret_cast<uintptr_t>(x) & 15)
         return MHD_ERR_ARG;  // rows are read as 16-byte chunks
-    k_colsum<<<blocks, threads, 0, s>>>(static_cast<const bf16*>(x), channels, (size_t)count, scratch);
+    mhd::launch_after(k_colsum, blocks, threads, 0, s, static_cast<const bf16*>(x), channels, (size_t)count, scratch);
     if (cudaGetLastError() != cudaSuccess)
         return MHD_ERR_CUDA;
-    k_sum_parts<<<(unsigned)((nout + 31) / 32), kSumWarps * 32, 0, s>>>(scratch, blocks, (size_t)channels,
-                                                                        (size_t)nout, out);
+    mhd::launch_after(k_sum_parts, (unsigned)((nout + 31) / 32), kSumWarps * 32, 0, s, scratch, blocks,
+        (size_t)channels, (size_t)nout, out);
     return st(cudaGetLastError());
 }
 
@@ -1628,14 +1642,15 @@ extern "C" MHD_API int mhd_cl_loss(const float* out, const void* target, void* d
     const size_t nv = (size_t)nb * n * n * n;
     const float gscale = 2.0f / (8.0f * (float)nv);
     const unsigned blocks = 512;
-    k_loss1<<<blocks, 256, 0, s>>>(out, static_cast<const bf16*>(target), static_cast<bf16*>(dout), rb_scratch,
-                                   loss_scratch, nb, n, gscale);
+    mhd::launch_after(k_loss1, blocks, 256, 0, s, out, static_cast<const bf16*>(target), static_cast<bf16*>(dout),
+        rb_scratch, loss_scratch, nb, n, gscale);
     if (cudaGetLastError() != cudaSuccess)
         return MHD_ERR_CUDA;
-    k_loss2<<<blocks_for(nv, 256), 256, 0, s>>>(rb_scratch, static_cast<bf16*>(dout), nb, n, gscale);
+    mhd::launch_after(k_loss2, blocks_for(nv, 256), 256, 0, s, rb_scratch, static_cast<bf16*>(dout), nb, n, gscale);
     if (cudaGetLastError() != cudaSuccess)
         return MHD_ERR_CUDA;
-    k_sum_parts<<<1, kSumWarps * 32, 0, s>>>(loss_scratch, (int)blocks, 1, 1, loss);  // sum of squares; /(8N) on the host
+    mhd::launch_after(k_sum_parts, 1, kSumWarps * 32, 0, s, loss_scratch, (int)blocks, 1, 1,
+        loss);  // sum of squares; /(8N) on the host
     return st(cudaGetLastError());
 }
 
@@ -1645,8 +1660,8 @@ extern "C" MHD_API int mhd_cl_features(const float* u, const float* b, int n, co
     if (!u || !b || n <= 0 || (!raw && !x) || (x && (!mean || !inv_std)))
         return MHD_ERR_ARG;
     const size_t nv = (size_t)n * n * n;
-    k_features<<<blocks_for(nv, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(u, b, n, mean, inv_std, raw,
-                                                                                   static_cast<bf16*>(x));
+    mhd::launch_after(k_features, blocks_for(nv, 256), 256, 0, static_cast<cudaStream_t>(stream), u, b, n, mean,
+        inv_std, raw, static_cast<bf16*>(x));
     return st(cudaGetLastError());
 }
 
@@ -1690,9 +1705,20 @@ extern "C" MHD_API int mhd_cl_diff(const float* ua, const float* ba, const float
     return st(cudaGetLastError());
 }
 
+// clears the flags and the sums of a correction (one launch in place of two memsets)
+__global__ void k_apply_begin(int* flags, double* esum)
+{
+    mhd::after_previous();
+    if (threadIdx.x < 4)
+        flags[threadIdx.x] = 0;
+    if (threadIdx.x < 8)
+        esum[threadIdx.x] = 0.0;
+}
+
 // between attempts: committed -> flags[1]; clear the failure bit and the energy sums
 __global__ void k_apply_next(int* flags, double* esum)
 {
+    mhd::after_previous();
     flags[1] = flags[2];
     flags[0] = 0;
     esum[0] = esum[1] = 0.0;
@@ -1707,19 +1733,18 @@ extern "C" MHD_API int mhd_cl_apply(float* u, float* b, const float* out, int n,
         return MHD_ERR_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t nv = (size_t)n * n * n;
-    if (cudaMemsetAsync(flags, 0, 4 * sizeof(int), s) != cudaSuccess ||
-        cudaMemsetAsync(esum, 0, 8 * sizeof(double), s) != cudaSuccess)
-        return MHD_ERR_CUDA;
+    mhd::launch_after(k_apply_begin, 1, 32, 0, s, flags, esum);
     const unsigned blocks = blocks_for(nv, 256);
     const unsigned rblocks = blocks < 2u * (unsigned)sms() ? blocks : 2u * (unsigned)sms();  // of the reductions
-    k_apply0<<<rblocks, 256, 0, s>>>(out, nv, esum, dt, dt_min);
+    mhd::launch_after(k_apply0, rblocks, 256, 0, s, out, nv, esum, dt, dt_min);
     for (int a = 0; a < 3; a++) {  // the full correction, else half, else a quarter, else none
         if (a)
-            k_apply_next<<<1, 1, 0, s>>>(flags, esum);
-        k_apply1<<<rblocks, 256, 0, s>>>(u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp, esum, flags, dt,
-                                        dt_min);
-        k_apply2<<<blocks, 256, 0, s>>>(u_tmp, b_tmp, n, flags, dt, dt_min);
-        k_apply3<<<blocks, 256, 0, s>>>(u, b, u_tmp, b_tmp, nv, flags, esum, ecap, fallbacks, a == 2, dt, dt_min);
+            mhd::launch_after(k_apply_next, 1, 1, 0, s, flags, esum);
+        mhd::launch_after(k_apply1, rblocks, 256, 0, s, u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp,
+            esum, flags, dt, dt_min);
+        mhd::launch_after(k_apply2, blocks, 256, 0, s, u_tmp, b_tmp, n, flags, dt, dt_min);
+        mhd::launch_after(k_apply3, blocks, 256, 0, s, u, b, u_tmp, b_tmp, nv, flags, esum, ecap, fallbacks,
+            a == 2, dt, dt_min);
     }
     return st(cudaGetLastError());
 }
@@ -1730,8 +1755,8 @@ extern "C" MHD_API int mhd_cl_adamw(float* p, const float* g, float* m, float* v
     if (!p || !g || !m || !v || count <= 0 || step <= 0)
         return MHD_ERR_ARG;
     const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-    k_adamw<<<blocks_for((size_t)count, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        p, g, m, v, (size_t)count, lr, beta1, beta2, eps, wd, c1, c2);
+    mhd::launch_after(k_adamw, blocks_for((size_t)count, 256), 256, 0, static_cast<cudaStream_t>(stream), p, g, m,
+        v, (size_t)count, lr, beta1, beta2, eps, wd, c1, c2);
     return st(cudaGetLastError());
 }
 
@@ -1742,7 +1767,7 @@ extern "C" MHD_API int mhd_cl_pack(const float* w, int cout_real, int cin_real, 
         (!w_fwd && !w_dgrad))
         return MHD_ERR_ARG;
     const size_t tot = (size_t)cout_pad * taps * cin_pad;
-    k_pack<<<blocks_for(tot, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, cout_real, cin_real, taps, cout_pad, cin_pad, static_cast<bf16*>(w_fwd), static_cast<bf16*>(w_dgrad));
+    mhd::launch_after(k_pack, blocks_for(tot, 256), 256, 0, static_cast<cudaStream_t>(stream), w, cout_real,
+        cin_real, taps, cout_pad, cin_pad, static_cast<bf16*>(w_fwd), static_cast<bf16*>(w_dgrad));
     return st(cudaGetLastError());
 }

@@ -95,8 +95,7 @@ static cudaError_t launch_fx2(const FluidxArgs& a, cudaStream_t s)
             return e;
         smem = fluidx_sweep_smem_bytes(n);
     }
-    k_fluidx2<R, EX, C, T, AX><<<grid, a.P * T, smem, s>>>(a, tm);
-    return cudaGetLastError();
+    return launch_after(k_fluidx2<R, EX, C, T, AX>, grid, a.P * T, smem, s, a, tm);
 }
 
 // Sweep of the untransposed state along y or z (fused step, FP32): pencils
@@ -152,8 +151,8 @@ static cudaError_t fluidx_any(const FluidxArgs& a, cudaStream_t s)
         if (e != cudaSuccess)
             return e;
         dim3 grid(a.ny / a.P, a.nz, a.bs.count);
-        k_fluidx<RR, EX><<<grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx, a.P) * sizeof(RR), s>>>(a);
-        return cudaGetLastError();
+        return launch_after(k_fluidx<RR, EX>, grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx,
+            a.P) * sizeof(RR), s, a);
     }
 }
 
@@ -267,6 +266,10 @@ static bool plan_advect3(int nx, int ny, int nz, bool aligned, A3Plan& p, int ax
     }
     if (!p.J)
         return false;
+    // a small grid: fewer pencils per CTA until every SM has one (32^3: 256 CTAs of 4 pencils, not 64 of 16)
+    for (int j = p.J - 1; !jt && j >= 1 && (long long)(ny / p.J) * nz * boxes < 152; j--)
+        if (ny % j == 0)
+            p.J = j;
     const int kt = tune_value(TUNE_ADVECT_K);
     p.K = 1;
     for (int k = 1; k <= nz && k <= 64; k++) {
@@ -288,9 +291,8 @@ static cudaError_t launch_ad3(const AdvectArgs& a, cudaStream_t s)
         return e;
     const int nj = (AX == 0) ? a.ny : a.nx, nk = (AX == 2) ? a.ny : a.nz;
     dim3 grid(nj / a.P, nk / a.K, a.bs.count);
-    k_advect3<EX, C, T, NS, AX, WU><<<grid, advect3_threads(a.P, T),
-                                      advect3_smem_floats(a.P, C * T, NS, AX, WU ? 2 : 5) * sizeof(float), s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_advect3<EX, C, T, NS, AX, WU>, grid, advect3_threads(a.P, T),
+                        advect3_smem_floats(a.P, C * T, NS, AX, WU ? 2 : 5) * sizeof(float), s, a);
 }
 
 template <int C, int NS, int AX = 0, bool WU = false>
@@ -382,8 +384,7 @@ static cudaError_t launch_ad4(const AdvectArgs& a, cudaStream_t s)
     if (ctas > cap)
         ctas = cap;
     dim3 grid((unsigned)ctas, 1, a.bs.count);
-    k_advect4<EX, KT, NS, WU><<<grid, advect4_threads(KT), smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_advect4<EX, KT, NS, WU>, grid, advect4_threads(KT), smem, s, a);
 }
 
 static cudaError_t advect_x4(const AdvectArgs& a, const A4Plan& p, cudaStream_t s)
@@ -476,8 +477,7 @@ static cudaError_t launch_ad6(const AdvectArgs& a, int K, cudaStream_t s)
             return e;
     }
     dim3 grid(a.ny / J, (a.kcount ? a.kcount : a.nz) / K, a.bs.count);
-    k_advect6<EX, C, J, SW><<<grid, advect6_threads(J), advect6_smem_bytes(C * 32, J), s>>>(b, wmap);
-    return cudaGetLastError();
+    return launch_after(k_advect6<EX, C, J, SW>, grid, advect6_threads(J), advect6_smem_bytes(C * 32, J), s, b, wmap);
 }
 
 static cudaError_t advect_x6(const AdvectArgs& a, const A6Plan& p, cudaStream_t s)
@@ -552,8 +552,7 @@ static cudaError_t launch_ad5(const AdvectArgs& a, cudaStream_t s)
     const long long cap = (work / 8 > 0) ? work / 8 : 1;
     if (ctas > cap)
         ctas = cap;
-    k_advect5<EX, KT, NS, AX, WU><<<dim3((unsigned)ctas, 1, 1), advect5_threads(KT), smem, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_advect5<EX, KT, NS, AX, WU>, dim3((unsigned)ctas, 1, 1), advect5_threads(KT), smem, s, a);
 }
 
 template <int AX, bool WU>
@@ -587,8 +586,8 @@ static cudaError_t launch_ad2(const AdvectArgs& a, cudaStream_t s)
     if (e != cudaSuccess)
         return e;
     dim3 grid(a.ny / a.P, a.nz, a.bs.count);
-    k_advect2<R, EX, C, T><<<grid, advect2_threads(a.P, T), advect2_smem_elems(a.nx, a.P) * sizeof(R), s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_advect2<R, EX, C, T>, grid, advect2_threads(a.P, T), advect2_smem_elems(a.nx,
+        a.P) * sizeof(R), s, a);
 }
 
 static cudaError_t advect(const AdvectArgs& in, cudaStream_t s)
@@ -675,8 +674,7 @@ static cudaError_t advect(const AdvectArgs& in, cudaStream_t s)
     if (threads < 128)
         threads = 128;
     dim3 grid(a.ny / a.P, a.nz, a.bs.count);
-    k_advect<R, EX><<<grid, threads, advect_smem_elems(a.nx, a.P) * sizeof(R), s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_advect<R, EX>, grid, threads, advect_smem_elems(a.nx, a.P) * sizeof(R), s, a);
 }
 
 // -------------------------------------------------------------- transposes
@@ -690,28 +688,16 @@ static cudaError_t transpose(const TransposeArgs& a, cudaStream_t s)
                              reinterpret_cast<uintptr_t>(a.uu) | reinterpret_cast<uintptr_t>(a.ub);
         if (a.nx % kT3 == 0 && na % kT3 == 0 && (al & 15) == 0) {  // bulk-TMA tiles
             dim3 grid(a.nx / kT3, na / kT3, nb * a.bs.count);
-            if (a.axis == 1)
-                k_transpose3<1><<<grid, 256, 0, s>>>(a);
-            else
-                k_transpose3<2><<<grid, 256, 0, s>>>(a);
-            return cudaGetLastError();
+            return launch_after(a.axis == 1 ? k_transpose3<1> : k_transpose3<2>, grid, 256, 0, s, a);
         }
         if (a.nx % 16 == 0 && na % 16 == 0 && (al & 15) == 0) {  // bulk-TMA tiles of 16 cells
             dim3 grid(a.nx / 16, na / 16, nb * a.bs.count);
-            if (a.axis == 1)
-                k_transpose3<1, 16><<<grid, 256, 0, s>>>(a);
-            else
-                k_transpose3<2, 16><<<grid, 256, 0, s>>>(a);
-            return cudaGetLastError();
+            return launch_after(a.axis == 1 ? k_transpose3<1, 16> : k_transpose3<2, 16>, grid, 256, 0, s, a);
         }
     }
     constexpr int T = TTile<R>::E;
     dim3 grid((a.nx + T - 1) / T, (na + T - 1) / T, nb * a.bs.count);
-    if (a.axis == 1)
-        k_transpose<1, R><<<grid, 256, 0, s>>>(a);
-    else
-        k_transpose<2, R><<<grid, 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(a.axis == 1 ? k_transpose<1, R> : k_transpose<2, R>, grid, 256, 0, s, a);
 }
 
 // ------------------------------------------------------------------ calcfl
@@ -721,9 +707,8 @@ static cudaError_t calcfl(const void* u, const void* b, size_t ncell, size_t cel
 {
     const int blocks = (int)((ncell + 255) / 256);
     *nparts = blocks;
-    k_calcfl<R, EX><<<dim3(blocks, bs.count), 256, 0, s>>>(static_cast<const R*>(u), static_cast<const R*>(b), ncell,
-                                                           cell0, static_cast<CflPart<R>*>(part), bs);
-    return cudaGetLastError();
+    return launch_after(k_calcfl<R, EX>, dim3(blocks, bs.count), 256, 0, s, static_cast<const R*>(u),
+                        static_cast<const R*>(b), ncell, cell0, static_cast<CflPart<R>*>(part), bs);
 }
 
 static cudaError_t cfl_finalize(const CflFinalizeArgs& in, cudaStream_t s)
@@ -732,16 +717,15 @@ static cudaError_t cfl_finalize(const CflFinalizeArgs& in, cudaStream_t s)
     if (a.bs.count == 1 && a.scratch && a.nparts > kCflReduceMin) {
         int g = (a.nparts + 511) / 512;
         g = g < kCflReduceCtas ? g : kCflReduceCtas;
-        k_cfl_reduce<R><<<g, 256, 0, s>>>(static_cast<const CflPart<R>*>(a.part), a.nparts,
-                                          static_cast<CflPart<R>*>(a.scratch));
-        const cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_after(k_cfl_reduce<R>, g, 256, 0, s, static_cast<const CflPart<R>*>(a.part),
+            a.nparts,
+                                           static_cast<CflPart<R>*>(a.scratch));
         if (e != cudaSuccess)
             return e;
         a.part = a.scratch;
         a.nparts = g;
     }
-    k_cfl_finalize<R, EX><<<a.bs.count, 1024, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_after(k_cfl_finalize<R, EX>, a.bs.count, 1024, 0, s, a);
 }
 
 static cudaError_t divb(const void* b, int nx, int ny, int nz, double* part, int* nparts, cudaStream_t s)
@@ -891,8 +875,7 @@ static cudaError_t fluidx_multi(const FluidxArgs* in, int nseg, cudaStream_t s)
         m.nseg = nseg;
         if (total <= 0 || total >= (1LL << 31))
             return cudaErrorInvalidValue;
-        k_fluidx2_multi<R, EX><<<(unsigned)total, kMultiFxThreads, smem, s>>>(m);
-        return cudaGetLastError();
+        return launch_after(k_fluidx2_multi<R, EX>, (unsigned)total, kMultiFxThreads, smem, s, m);
     } else {
         (void)in, (void)nseg, (void)s;
         return cudaErrorNotSupported;
@@ -942,8 +925,7 @@ static cudaError_t advect_multi(const AdvectArgs* in, int nseg, cudaStream_t s)
         m.nseg = nseg;
         if (total <= 0 || total >= (1LL << 31))
             return cudaErrorInvalidValue;
-        k_advect6_multi<EX><<<(unsigned)total, advect6_threads(kMultiAdJ), smem, s>>>(m);
-        return cudaGetLastError();
+        return launch_after(k_advect6_multi<EX>, (unsigned)total, advect6_threads(kMultiAdJ), smem, s, m);
     } else {
         (void)in, (void)nseg, (void)s;
         return cudaErrorNotSupported;
@@ -977,11 +959,8 @@ static cudaError_t transpose_multi(const TransposeArgs* in, int nseg, cudaStream
         m.nseg = nseg;
         if (total <= 0 || total >= (1LL << 31))
             return cudaErrorInvalidValue;
-        if (axis == 1)
-            k_transpose_multi<1><<<(unsigned)total, 256, kMultiTransposeSmem, s>>>(m);
-        else
-            k_transpose_multi<2><<<(unsigned)total, 256, kMultiTransposeSmem, s>>>(m);
-        return cudaGetLastError();
+        return launch_after(axis == 1 ? k_transpose_multi<1> : k_transpose_multi<2>, (unsigned)total, 256,
+            kMultiTransposeSmem, s, m);
     } else {
         (void)in, (void)nseg, (void)s;
         return cudaErrorNotSupported;
@@ -1003,8 +982,7 @@ static cudaError_t finalize_multi(const CflFinalizeArgs* in, int nseg, cudaStrea
         total += in[i].bs.count;
     }
     m.nseg = nseg;
-    k_cfl_finalize_multi<R, EX><<<(unsigned)total, 1024, 0, s>>>(m);
-    return cudaGetLastError();
+    return launch_after(k_cfl_finalize_multi<R, EX>, (unsigned)total, 1024, 0, s, m);
 }
 
 static const KernelSet kSet = {(int)sizeof(R), EX ? 1 : 0, fluidx, advect, transpose, calcfl, cfl_finalize, divb,

@@ -114,6 +114,7 @@ __host__ __device__ inline size_t advect2_smem_elems(int n, int P)
 template <typename R, bool EX, int C, int T>
 __global__ void __launch_bounds__(512) k_advect2(AdvectArgs a)
 {
+    after_previous();
     select_box(a, blockIdx.z);
     using W = wide_t<R, EX>;
     constexpr int n = C * T;

@@ -56,6 +56,7 @@ __host__ __device__ inline size_t advect3_smem_floats(int J, int n, int NS, int 
 template <bool EX, int C, int T, int NS, int AX = 0, bool WU = false>
 __global__ void __launch_bounds__(384) k_advect3(AdvectArgs a)
 {
+    after_previous();
     select_box(a, blockIdx.z);
     using R = float;
     constexpr int n = C * T;
@@ -200,6 +201,8 @@ __global__ void __launch_bounds__(384) k_advect3(AdvectArgs a)
     const float* b1s = static_cast<const float*>(a.b1_src);
     float* bo = static_cast<float*>(a.b_out);
     for (int k = k0; k < k0 + K; k++) {
+        if (k + 1 == k0 + K)
+            before_next();
         const int sk = slot_of(k), sk1 = slot_of(k + 1);
         if (NS >= 3 && k + 2 <= k0 + K) {  // plane k-1's slot is free
             fence_proxy_async_smem();

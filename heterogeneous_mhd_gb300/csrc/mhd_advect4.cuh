@@ -186,6 +186,7 @@ __host__ __device__ constexpr int advect4_min_ctas(int KT, int NS)
 template <bool EX, int KT, int NS, bool WU = false>
 __global__ void __launch_bounds__((KT + 1) * 32, advect4_min_ctas(KT, NS)) k_advect4(AdvectArgs a)
 {
+    after_previous();
     static_assert(NS == 2 || NS == 3, "two or three chunk buffers");
     select_box(a, blockIdx.z);
     constexpr int NW = KT + 1;                            // warps

@@ -63,6 +63,7 @@ __host__ __device__ inline size_t advect5_smem_bytes(int KT, int NS, bool wu = f
 template <bool EX, int KT, int NS, int AX, bool WU = false>
 __global__ void __launch_bounds__((KT + 1) * 32, advect4_min_ctas(KT, NS)) k_advect5(AdvectArgs a)
 {
+    after_previous();
     static_assert(AX == 1 || AX == 2, "sweeps along y or z");
     static_assert(NS == 2 || NS == 3, "two or three chunk buffers");
     select_box(a, blockIdx.z);

@@ -198,6 +198,8 @@ __device__ __forceinline__ void advect6_body(AdvectArgs a, const CUtensorMap& wm
     }
 
     for (int k = k0; k < k0 + K; k++) {
+        if (k + 1 == k0 + K)
+            before_next();
         const int s = slot_of(k + 1);
         float* const fax = FAx + ((k - k0) & 1) * (J + 1) * n;
         // ---- A row (j, k) from the carried inputs
@@ -267,6 +269,7 @@ template <bool EX, int C, int J, bool SW = false>
 __global__ void __launch_bounds__((J + 1) * 32, advect6_min_ctas(J))
     k_advect6(AdvectArgs a, const __grid_constant__ CUtensorMap wmap)
 {
+    after_previous();
     advect6_body<EX, C, J, SW, 32>(a, wmap, HwBlock{});
 }
 

@@ -479,6 +479,7 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
         }
     }
 
+    before_next();
     // ---- optional calcfl epilogue on the new state (face b at (j,k)); x sweep only
     if (AX == 0 && a.cfl_part) {
         const R* bj = sb + (size_t)lp * SB + (size_t)i0 * 3;
@@ -578,6 +579,7 @@ template <typename R, bool EX, int C, int T, int AX = 0>
 __global__ void __launch_bounds__(AX ? kSweepP * T : 256, AX ? (T <= 64 ? 3 : 1) : 0)
     k_fluidx2(FluidxArgs a, const __grid_constant__ SweepMaps tm)
 {
+    after_previous();
     fluidx2_body<R, EX, C, T, AX>(a, &tm, HwBlock{});
 }
 

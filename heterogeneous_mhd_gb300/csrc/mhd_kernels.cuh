@@ -240,6 +240,7 @@ __host__ __device__ inline size_t fluidx_smem_elems(int n, int P)
 template <typename R, bool EX>
 __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
 {
+    after_previous();
     select_box(a, blockIdx.z, sizeof(CflPart<R>), gridDim.x * gridDim.y);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = a.nx, P = a.P;
@@ -459,6 +460,7 @@ __host__ __device__ inline size_t advect_smem_elems(int n, int P)
 template <typename R, bool EX>
 __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
 {
+    after_previous();
     select_box(a, blockIdx.z);
     using W = wide_t<R, EX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -696,6 +698,7 @@ __device__ __forceinline__ void transpose_tile(const TransposeArgs& a, R* su, R*
         ow[q] = (f >> 1) * SU + perm_u<AXIS>(f & 1);
     }
     __syncthreads();
+    before_next();
     // output: axis 1 -> dims (ny,nx,nz), cell (a, i, z); axis 2 -> dims (nz,ny,nx), cell (a, z, i)
 #pragma unroll
     for (int s = 0; s < RW; s++) {
@@ -723,6 +726,7 @@ __device__ __forceinline__ void transpose_tile(const TransposeArgs& a, R* su, R*
 template <int AXIS, typename R>
 __global__ void __launch_bounds__(256) k_transpose(TransposeArgs a)
 {
+    after_previous();
     constexpr int kTT = TTile<R>::E;
     __shared__ R su[kTT * (kTT * 5 + 5)];
     __shared__ R sb[kTT * (kTT * 3 + 3)];
@@ -735,12 +739,28 @@ __global__ void __launch_bounds__(256) k_transpose(TransposeArgs a)
 // copy_matrix (C/copy_matrix.c:9-38) as a vectorised device copy.
 static __global__ void __launch_bounds__(256) k_copy16(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16)
 {
+    after_previous();
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n16; e += (size_t)gridDim.x * blockDim.x)
         dst[e] = src[e];
 }
 
+// u and b in one launch (a small state's copies are launch latency)
+static __global__ void __launch_bounds__(256) k_copy16x2(const uint4* __restrict__ src0, uint4* __restrict__ dst0,
+                                                         size_t n0, const uint4* __restrict__ src1,
+                                                         uint4* __restrict__ dst1, size_t n1)
+{
+    after_previous();
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n0 + n1; e += (size_t)gridDim.x * blockDim.x) {
+        if (e < n0)
+            dst0[e] = src0[e];
+        else
+            dst1[e - n0] = src1[e - n0];
+    }
+}
+
 static __global__ void __launch_bounds__(256) k_copy4(const float* __restrict__ src, float* __restrict__ dst, size_t n4)
 {
+    after_previous();
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n4; e += (size_t)gridDim.x * blockDim.x)
         dst[e] = src[e];
 }
@@ -754,6 +774,7 @@ template <typename R, bool EX>
 __global__ void __launch_bounds__(256) k_calcfl(const R* __restrict__ u, const R* __restrict__ b, size_t ncell,
                                                 size_t cell0, CflPart<R>* part, BoxStrides bs)
 {
+    after_previous();
     __shared__ R rm[8];
     __shared__ int rn[8];
     // batched: box blockIdx.y, its partials after those of the boxes before it
@@ -810,6 +831,8 @@ template <typename R>
 __global__ void __launch_bounds__(256) k_cfl_reduce(const CflPart<R>* __restrict__ part, int nparts,
                                                     CflPart<R>* __restrict__ out)
 {
+    before_next();  // a few CTAs: the next grid spreads over the other SMs
+    after_previous();
     __shared__ R rm[8];
     __shared__ int rn[8];
     const int per = (nparts + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -946,6 +969,8 @@ __device__ __forceinline__ void cfl_finalize_body(CflFinalizeArgs a, const B& bl
 template <typename R, bool EX>
 __global__ void __launch_bounds__(1024) k_cfl_finalize(CflFinalizeArgs a)
 {
+    before_next();  // a few CTAs: the next grid spreads over the other SMs
+    after_previous();
     cfl_finalize_body<R, EX>(a, HwBlock{});
 }
 

@@ -67,6 +67,9 @@ int fluidx_pencils(int nx, int ny);
 int advect_pencils(int nx, int ny);
 
 cudaError_t launch_copy(const void* src, void* dst, size_t bytes, cudaStream_t s);
+// two copies, in one launch where both are of aligned 16-byte pieces; returns the launches made
+int launch_copy2(const void* src0, void* dst0, size_t bytes0, const void* src1, void* dst1, size_t bytes1,
+                 cudaStream_t s, cudaError_t* e);
 
 // Raise a kernel's dynamic shared-memory limit to the device's opt-in maximum
 // minus its static shared memory (once per kernel).  Kernels that stage all

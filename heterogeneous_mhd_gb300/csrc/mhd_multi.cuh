@@ -116,6 +116,7 @@ __device__ __forceinline__ VBlock multi_block(const SegGrid& g)
 template <typename R, bool EX>
 __global__ void __launch_bounds__(kMultiFxThreads) k_fluidx2_multi(const __grid_constant__ FluidxMulti m)
 {
+    after_previous();
     const int s = multi_seg(m.g, m.nseg);
     const VBlock blk = multi_block(m.g[s]);
     switch (m.g[s].kind) {
@@ -136,6 +137,7 @@ template <bool EX>
 __global__ void __launch_bounds__((kMultiAdJ + 1) * 32, 6)
     k_advect6_multi(const __grid_constant__ AdvectMulti m)
 {
+    after_previous();
     const int s = multi_seg(m.g, m.nseg);
     const VBlock blk = multi_block(m.g[s]);
     const CUtensorMap& wm = m.wmap[s];
@@ -157,6 +159,7 @@ constexpr size_t kMultiTransposeSmem = kT3SmemBytes;
 template <int AXIS>
 __global__ void __launch_bounds__(256, 6) k_transpose_multi(const __grid_constant__ TransposeMulti m)
 {
+    after_previous();
     extern __shared__ __align__(16) unsigned char tmul_raw[];
     float* const sm = reinterpret_cast<float*>(tmul_raw);
     const int s = multi_seg(m.g, m.nseg);
@@ -170,6 +173,8 @@ __global__ void __launch_bounds__(256, 6) k_transpose_multi(const __grid_constan
 template <typename R, bool EX>
 __global__ void __launch_bounds__(1024) k_cfl_finalize_multi(const __grid_constant__ FinalizeMulti m)
 {
+    before_next();
+    after_previous();
     const int s = multi_seg(m.g, m.nseg);
     cfl_finalize_body<R, EX>(m.a[s], multi_block(m.g[s]));
 }

@@ -20,6 +20,39 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Programmatic dependent launch.  Every kernel of a step is launched with
+// launch_after (below).  It begins with after_previous(), which waits until the
+// kernel before it has completed and its writes are visible (at once in a plain
+// launch); no global memory is touched before that.  Where a CTA has little left
+// to do it calls before_next(): once all CTAs have (or have ended), the next
+// kernel is brought in, so its launch overlaps this one's last stores.  Called
+// at the start instead, the next kernel's CTAs fill the SMs that happen to be free
+// first and a grid of less than a wave spreads unevenly.  Ten plain 64^3 steps / two
+// EXACT 96^3 / four 100x72x72 / four corrected 64^3: 1.02, 1.15, 1.08, 1.52 ms
+// without any of this, 1.11, 1.11, 1.02, 1.39 with before_next at the start, 1.02,
+// 1.11, 1.03, 1.33 as it is.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void before_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A launch that may start while the one before it in the stream drains; the
+// kernel begins with after_previous().  Captured into a graph it becomes a
+// programmatic edge.
+template <typename... P, typename... A>
+static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
 {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

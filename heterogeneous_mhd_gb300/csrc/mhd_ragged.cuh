@@ -249,6 +249,7 @@ __device__ __forceinline__ void rag_cell_flux(const float q[5], const float f[3]
 template <bool EX, int C, int D>
 __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagShape sh, int pb)
 {
+    after_previous();
     using R = float;
     select_box(a, blockIdx.z, sizeof(CflPart<R>), gridDim.x * gridDim.y);
     extern __shared__ __align__(16) float rag_smem[];
@@ -413,6 +414,7 @@ __global__ void __launch_bounds__(kRagThreads) k_fluidx_rag(FluidxArgs a, RagSha
             }
         }
 
+    before_next();
     // ---- optional calcfl epilogue on the new state (face b at (j,k))
     if (a.cfl_part) {
         const R* bj = sb + lp * SB + 3 * i0;
@@ -543,6 +545,7 @@ __device__ __forceinline__ void rag_tvdb_row(const RagGroup<C, D>& g, const floa
 template <bool EX, int C, int D, bool WU>
 __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, int pb)
 {
+    after_previous();
     select_box(a, blockIdx.z);
     extern __shared__ __align__(16) float rag_smem[];
     const int n = a.nx, ny = a.ny, nz = a.nz, J = a.P, tid = threadIdx.x, tc = sh.T * C;
@@ -642,6 +645,8 @@ __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, i
     issue(k0 + 1);
     issue(k0 + 2);
     for (int k = k0; k < k1; k++) {
+        if (k + 1 == k1)
+            before_next();
         float* const fax = FAx + (k & 1) * (J + 1) * SF;
         float FA[C], bA[C], FBn[C], b3n[C], rc[C], mc[C], bb[3 * C];
         rag_tvdb_row<EX, C, D>(g, vA, b2c, dt, seam, FA, bA);
@@ -723,8 +728,7 @@ static cudaError_t launch_fx_rag(const FluidxArgs& a, const RagShape& sh, int pb
     if (e != cudaSuccess)
         return e;
     const dim3 grid((a.ny + a.P - 1) / a.P, a.nz, a.bs.count);
-    k_fluidx_rag<EX, C, D><<<grid, a.P * sh.G, rag_fluidx_smem(sh), s>>>(a, sh, pb);
-    return cudaGetLastError();
+    return launch_after(k_fluidx_rag<EX, C, D>, grid, a.P * sh.G, rag_fluidx_smem(sh), s, a, sh, pb);
 }
 
 template <bool EX, int C, int D>
@@ -738,11 +742,8 @@ static cudaError_t launch_ad_rag(const AdvectArgs& a, const RagShape& sh, int pb
     const dim3 grid((a.ny + a.P - 1) / a.P, (a.nz + a.K - 1) / a.K, a.bs.count);
     const int nt = ((a.P + 1) * sh.G + 31) / 32 * 32;  // whole warps: groups past the halo pencil's repeat it
     const size_t smem = rag_advect_smem(sh, a.P);
-    if (wu)
-        k_advect_rag<EX, C, D, true><<<grid, nt, smem, s>>>(a, sh, pb);
-    else
-        k_advect_rag<EX, C, D, false><<<grid, nt, smem, s>>>(a, sh, pb);
-    return cudaGetLastError();
+    return launch_after(wu ? k_advect_rag<EX, C, D, true> : k_advect_rag<EX, C, D, false>, grid, nt, smem, s, a,
+        sh, pb);
 }
 
 template <bool EX>

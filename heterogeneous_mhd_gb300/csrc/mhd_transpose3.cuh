@@ -91,6 +91,7 @@ __device__ __forceinline__ void transpose3_body(TransposeArgs a, float* __restri
     // whole CTA leaves before writing from unfilled shared memory
     if (!__syncthreads_and(mbar_wait_bounded(&bar, 0, a.err)))
         return;
+    before_next();
 
     float* uo = static_cast<float*>(a.u_out);
     float* bo = static_cast<float*>(a.b_out);
@@ -121,6 +122,7 @@ __device__ __forceinline__ void transpose3_body(TransposeArgs a, float* __restri
 template <int AXIS, int E = kT3>
 __global__ void __launch_bounds__(256) k_transpose3(TransposeArgs a)
 {
+    after_previous();
     __shared__ __align__(16) float su[E * T3Tile<E>::SU];
     __shared__ __align__(16) float sb[E * T3Tile<E>::SB];
     transpose3_body<AXIS, E>(a, su, sb, HwBlock{});
