@@ -14,6 +14,7 @@ not been built (``python -c "import __graft_entry__ as g; g.build()"``).
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from pathlib import Path
 
 import numpy as np
@@ -153,10 +154,12 @@ def _ptr(a) -> int:
         if not a.flags["C_CONTIGUOUS"]:
             raise ValueError("arrays must be contiguous")
         return a.ctypes.data
-    if hasattr(a, "data_ptr"):
-        if hasattr(a, "is_contiguous") and not a.is_contiguous():
+    ptr = getattr(a, "data_ptr", None)
+    if ptr is not None:
+        contiguous = getattr(a, "is_contiguous", None)
+        if contiguous is not None and not contiguous():
             raise ValueError("tensors must be contiguous")
-        return a.data_ptr()
+        return ptr()
     if isinstance(a, int):
         return a
     raise TypeError(f"unsupported array type {type(a)!r}")
@@ -167,7 +170,9 @@ def _check(status: int, what: str) -> None:
         raise MhdError(status, what)
 
 
+@functools.lru_cache(maxsize=64)
 def _dims(nx, ny, nz):
+    """The dimensions as the C surface takes them, by pointer (read only there)."""
     return C.byref(C.c_int(nx)), C.byref(C.c_int(ny)), C.byref(C.c_int(nz))
 
 

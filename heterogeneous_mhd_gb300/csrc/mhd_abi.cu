@@ -414,6 +414,20 @@ static int op_copy(mhd_ctx* c, const void* src, void* dst, size_t bytes)
     return MHD_OK;
 }
 
+// copy_matrix of u and b
+static int op_copy2(mhd_ctx* c, const void* su, void* du, size_t bu, const void* sb, void* db, size_t bb)
+{
+    if (su == du || sb == db) {
+        MHD_TRY(op_copy(c, su, du, bu));
+        return op_copy(c, sb, db, bb);
+    }
+    cudaError_t e = cudaSuccess;
+    KTimer kt(c, MHD_K_COPY);
+    c->launch_count += launch_copy2(su, du, bu, sb, db, bb, c->stream, &e) - 1;
+    CUDA_TRY(e);
+    return MHD_OK;
+}
+
 // First CFL pass into `dst` (grown to fit); returns the partial count in *np.
 static int op_calcfl_partials(mhd_ctx* c, DevBuf& dst, const void* u, const void* b, size_t cells, int* np)
 {
@@ -511,8 +525,7 @@ extern "C" MHD_API int mhd_op_copy(mhd_ctx* c, const void* u, const void* b, voi
     if (!c || !u || !b || !uu || !ub || nx < 0 || ny < 0 || nz < 0)
         return set_err(MHD_ERR_ARG);
     const size_t cells = (size_t)nx * ny * nz;
-    MHD_TRY(set_err(op_copy(c, u, uu, cells * 5 * c->elem)));
-    return set_err(op_copy(c, b, ub, cells * 3 * c->elem));
+    return set_err(op_copy2(c, u, uu, cells * 5 * c->elem, b, ub, cells * 3 * c->elem));
 }
 
 static int read_clock(mhd_ctx* c, const void* clock, double out[4])
@@ -542,10 +555,10 @@ static int calcfl_sync(mhd_ctx* c, const void* u, const void* b, int nx, int ny,
     MHD_TRY(op_calcfl_partials(c, c->opart, u, b, cells, &np));
     MHD_TRY(op_finalize(c, c->opart.p, c->opclock.p, np, u, b, nx, ny, nz, 0.0, 0));
     double clk[4];
-    MHD_TRY(read_clock(c, c->opclock.p, clk));
-    *inv = clk[3];
     int herr = 0;
-    CUDA_TRY(cudaMemcpy(&herr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpyAsync(&herr, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    MHD_TRY(read_clock(c, c->opclock.p, clk));  // waits for both
+    *inv = clk[3];
     if (herr & DEVERR_NONFINITE) {
         CUDA_TRY(cudaMemsetAsync(c->err_dev, 0, sizeof(int), c->stream));
         CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1533,8 +1546,7 @@ extern "C" MHD_API void copy_matrix(float* u, float* b, int* nx, int* ny, int* n
                    {update_b, cells * 12, false, true}};
     if (set_err(stage_in(c, args, 4)) != MHD_OK)
         return;
-    if (set_err(op_copy(c, args[0].dev, args[2].dev, cells * 20)) != MHD_OK ||
-        set_err(op_copy(c, args[1].dev, args[3].dev, cells * 12)) != MHD_OK)
+    if (set_err(op_copy2(c, args[0].dev, args[2].dev, cells * 20, args[1].dev, args[3].dev, cells * 12)) != MHD_OK)
         return;
     set_err(stage_out(c, args, 4));
 }
@@ -1655,8 +1667,7 @@ static void cuda_transpose(int axis, float* ut, float* bt, float* u, float* b, c
     // like the reference's wrappers (Cuda/cuda_transpose12.cu:30-34), the
     // transposed state is copied back, so u and b hold it on return as well
     const size_t cells = (size_t)(*h_nx) * (*h_ny) * (*h_nz);
-    if (set_err(op_copy(c, ut, u, cells * 5 * sizeof(float))) != MHD_OK ||
-        set_err(op_copy(c, bt, b, cells * 3 * sizeof(float))) != MHD_OK)
+    if (set_err(op_copy2(c, ut, u, cells * 5 * sizeof(float), bt, b, cells * 3 * sizeof(float))) != MHD_OK)
         return;
     set_err(cudaStreamSynchronize(c->stream) == cudaSuccess ? MHD_OK : MHD_ERR_CUDA);
 }
