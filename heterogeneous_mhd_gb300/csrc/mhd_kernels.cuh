@@ -173,30 +173,35 @@ __device__ __forceinline__ R warp_max(R x)
 }
 
 // Max over the n cells of the caller's pencil, starting from 0 and skipping
-// NaN (find_max, C/mhdflux.c:61-72).  Contains one __syncthreads; red must not
-// be read by a previous call that is not separated by another barrier.
-template <typename R>
-__device__ __forceinline__ R pencil_max(R x, R* red, int n, int lp)
+// NaN (find_max, C/mhdflux.c:61-72); the values are non-negative, so their bits
+// are ordered as they are.  Contains one __syncthreads; red must not be read by a
+// previous call that is not separated by another barrier.
+__device__ __forceinline__ double pencil_max64(double x, double* red, int n, int lp)
 {
+    using U = unsigned long long;
+    auto top = [](U a, U b) { return a > b ? a : b; };
+    U m = (U)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+    m = m > 0x7ff0000000000000ULL ? 0 : m;  // NaN
+    U* r = reinterpret_cast<U*>(red);
+    U c = 0;
     if ((n & 31) == 0) {
-        R m = warp_max(x);
-        const int w = threadIdx.x >> 5;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            m = top(m, __shfl_xor_sync(0xffffffffu, m, o));
         if ((threadIdx.x & 31) == 0)
-            red[w] = m;
+            r[threadIdx.x >> 5] = m;
         __syncthreads();
         const int wpp = n >> 5, w0 = lp * wpp;
-        R c = R(0);
         for (int s = 0; s < wpp; s++)
-            c = fmax(c, red[w0 + s]);
-        return c;
+            c = top(c, r[w0 + s]);
+    } else {
+        r[threadIdx.x] = m;
+        __syncthreads();
+        const U* row = r + lp * n;
+        for (int s = 0; s < n; s++)
+            c = top(c, row[s]);
     }
-    red[threadIdx.x] = x;
-    __syncthreads();
-    R c = R(0);
-    const R* row = red + lp * n;
-    for (int s = 0; s < n; s++)
-        c = fmax(c, row[s]);
-    return c;
+    return __longlong_as_double((long long)c);
 }
 
 // --------------------------------------------------------------- staging
@@ -237,6 +242,8 @@ __host__ __device__ inline size_t fluidx_smem_elems(int n, int P)
 // neighbour stencil is exchanged through shared memory between barriers.
 // Optionally (cfl_part != nullptr) the epilogue evaluates calcfl's per-cell
 // speed on the new u and the face b, and writes one partial max per CTA.
+// FP64 only (the FP32 lengths without a fixed engine: mhd_ragged.cuh), bound by
+// the FP64 pipe: one thread per cell and plain exchanges cost nothing beside it.
 template <typename R, bool EX>
 __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
 {
@@ -303,51 +310,47 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
         const R* bj = sb + 3 * lp * n;
         const R* bjp = sb + 3 * (lp + 1) * n;
         const R* bkp = sbk + 3 * lp * n;
-        const R h0 = R(0.5) * bj[3 * i], h0p = R(0.5) * bj[3 * ip];
-        f[0] = h0 + h0p;
-        f[1] = R(0.5) * bj[3 * i + 1] + bjp[3 * i + 1] / R(2);
-        f[2] = R(0.5) * bj[3 * i + 2] + bkp[3 * i + 2] / R(2);
+        f[0] = R(0.5) * __dadd_rn(bj[3 * i], bj[3 * ip]);
+        f[1] = R(0.5) * __dadd_rn(bj[3 * i + 1], bjp[3 * i + 1]);
+        f[2] = R(0.5) * __dadd_rn(bj[3 * i + 2], bkp[3 * i + 2]);
     }
 
+    // Fluxes are kept undivided (2 flux, 2 dfrm, 2 dflm), the half goes into the step.
     // ---- stage 1 (C/tvd1.c:33-49)
     R v[5], ci, fr[5], flux[5], u1[5];
-    cell_flux<R, EX>(q, f, v, ci);
-    R c = pencil_max<R>(ci, red, n, lp);
-    scale_flux<R, EX>(v, c);
+    cell_flux64(q, f, v, ci);
+    R c = pencil_max64(ci, red, n, lp);
+    scale_flux<R, true>(v, c);
 #pragma unroll
     for (int s = 0; s < 5; s++) {
-        const R wr = lin<R, EX>(R(1), q[s], R(1), v[s]);
-        const R wl = lin<R, EX>(R(1), q[s], R(-1), v[s]);
-        fr[s] = scale0<R, EX>(c, wr);
+        fr[s] = scale64(c, __dadd_rn(q[s], v[s]));
         if (act)
-            xa[5 * me + s] = scale0<R, EX>(c, wl);  // fl(i-1) = c*wl(i)
+            xa[5 * me + s] = scale64(c, __dsub_rn(q[s], v[s]));  // fl(i-1) = c*wl(i)
     }
     __syncthreads();
 #pragma unroll
     for (int s = 0; s < 5; s++) {
-        flux[s] = lin<R, EX>(R(0.5), fr[s], R(-0.5), xa[5 * mep + s]);
+        flux[s] = __dsub_rn(fr[s], xa[5 * mep + s]);
         if (act)
             xb[5 * me + s] = flux[s];
     }
     __syncthreads();
     {
-        const R hdt = R(-0.5) * dt;  // -1.0 * dt / 2.0 in double: exact
+        const R hdt = R(-0.25) * dt;
 #pragma unroll
         for (int s = 0; s < 5; s++)
-            u1[s] = lin<R, EX>(R(1), q[s], hdt, lin<R, EX>(R(1), flux[s], R(-1), xb[5 * mem + s]));
+            u1[s] = __dadd_rn(__dadd_rn(q[s], __dmul_rn(hdt, __dsub_rn(flux[s], xb[5 * mem + s]))), R(0));
     }
 
     // ---- stage 2 (C/tvd1.c:51-116)
-    cell_flux<R, EX>(u1, f, v, ci);
-    c = pencil_max<R>(ci, red, n, lp);
-    scale_flux<R, EX>(v, c);
+    cell_flux64(u1, f, v, ci);
+    c = pencil_max64(ci, red, n, lp);
+    scale_flux<R, true>(v, c);
     R g[5];
 #pragma unroll
     for (int s = 0; s < 5; s++) {
-        const R wr = lin<R, EX>(R(1), u1[s], R(1), v[s]);
-        const R wl = lin<R, EX>(R(1), u1[s], R(-1), v[s]);
-        fr[s] = scale0<R, EX>(c, wr);
-        g[s] = scale0<R, EX>(c, wl);
+        fr[s] = scale64(c, __dadd_rn(u1[s], v[s]));
+        g[s] = scale64(c, __dsub_rn(u1[s], v[s]));
         if (act) {
             xa[5 * me + s] = fr[s];
             xa[5 * (np + me) + s] = g[s];
@@ -357,9 +360,9 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
     R gp[5];
 #pragma unroll
     for (int s = 0; s < 5; s++) {
-        gp[s] = xa[5 * (np + mep) + s];                                   // fl(i) = g(i+1)
-        const R dfrm = lin<R, EX>(R(0.5), fr[s], R(-0.5), xa[5 * mem + s]);
-        const R dflm = lin<R, EX>(R(0.5), g[s], R(-0.5), gp[s]);
+        gp[s] = xa[5 * (np + mep) + s];  // fl(i) = g(i+1)
+        const R dfrm = __dsub_rn(fr[s], xa[5 * mem + s]);
+        const R dflm = __dsub_rn(g[s], gp[s]);
         if (act) {
             xb[5 * me + s] = dfrm;
             xb[5 * (np + me) + s] = dflm;
@@ -369,20 +372,19 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
 #pragma unroll
     for (int s = 0; s < 5; s++) {
         // dfrp(i) = dfrm(i+1), dflp(i) = dflm(i+1)
-        const R dfr = vanleer<R, EX>(xb[5 * mep + s], xb[5 * me + s]);
-        const R dfl = vanleer<R, EX>(xb[5 * (np + mep) + s], xb[5 * (np + me) + s]);
-        const R t1 = lin<R, EX>(R(1), fr[s], R(-1), gp[s]);
-        const R t2 = lin<R, EX>(R(1), dfr, R(-1), dfl);
-        flux[s] = lin<R, EX>(R(0.5), t1, R(0.5), t2);
+        const R dfr = vanleer64(xb[5 * mep + s], xb[5 * me + s]);
+        const R dfl = vanleer64(xb[5 * (np + mep) + s], xb[5 * (np + me) + s]);
+        flux[s] = __dadd_rn(__dsub_rn(fr[s], gp[s]), __dsub_rn(dfr, dfl));
         if (act)
             xa[5 * me + s] = flux[s];
     }
     __syncthreads();
     {
-        const R mdt = -dt;
+        const R mdt = R(-0.5) * dt;
 #pragma unroll
         for (int s = 0; s < 5; s++) {
-            const R un = lin<R, EX>(R(1), q[s], mdt, lin<R, EX>(R(1), flux[s], R(-1), xa[5 * mem + s]));
+            const R un =
+                __dadd_rn(__dadd_rn(q[s], __dmul_rn(mdt, __dsub_rn(flux[s], xa[5 * mem + s]))), R(0));
             q[s] = un;
             if (act)
                 su[5 * me + s] = un;  // own slot: no other thread reads su after staging
@@ -530,7 +532,7 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
     for (int it = threadIdx.x; it < items; it += blockDim.x) {
         const int r = it / n, i = it - r * n;
         const int ip = (i + 1 == n) ? 0 : i + 1;
-        const R vh = lin<R, EX>(R(0.5), VG[it], R(0.5), VG[r * n + ip]);
+        const R vh = tvdb_vh<R, EX>(VG[it], VG[r * n + ip]);
         VH[it] = vh;
         F1[it] = (vh > R(0)) ? T2[it] : T2[r * n + ip];
     }

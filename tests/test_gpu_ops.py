@@ -278,3 +278,29 @@ def test_exact_ops_wide_magnitudes_vs_oracle(shape, lo, hi, mhd, cuda, oracle32)
     assert bitwise_equal(out["fluidx_u"], uo)
     assert bitwise_equal(out["advect_b"], bo)
     assert out["calcfl"][0] == np.float32(ref_cfl)
+
+
+@pytest.mark.parametrize("shape", [(32, 8, 4), (20, 5, 3), (33, 4, 2), (64, 6, 3)])
+@pytest.mark.parametrize("lo,hi", [(-6, 2), (-200, 20)])
+def test_fp64_ops_wide_magnitudes_vs_oracle(shape, lo, hi, mhd, cuda, oracle64):
+    """The FP64 forms with fewer FP64 operations (halves moved, zeros' signs left to the
+    last sum, maxima and signs from the bits): bit for bit against the oracle on
+    momenta, energies and fields of 2^lo .. 2^hi with exact zeros mixed in."""
+    nx, ny, nz = shape
+    rng = np.random.default_rng(nx * 1000 + 7 * hi - lo)
+    nc = nx * ny * nz
+    u = rng.standard_normal((nc, 5)) * 2.0 ** rng.uniform(lo, hi, (nc, 5))
+    u[rng.random((nc, 5)) < 0.05] = 0
+    u[:, 0] = 2.0 ** rng.uniform(-3, 3, nc)
+    b = rng.standard_normal((nc, 3)) * 2.0 ** rng.uniform(lo, hi, (nc, 3))
+    b[rng.random((nc, 3)) < 0.05] = 0
+    u, b = u.ravel(), b.ravel()
+    bin_ = b * 0.75
+    uo, bo = np.full_like(u, 7), bin_.copy()
+    oracle64.fluidx(uo, b.copy(), nx, ny, nz, DT, u.copy(), b.copy())
+    oracle64.advectbyzx(u.copy(), bo, nx, ny, nz, DT, u.copy(), b.copy())
+    with mhd.Context(1, 1, 1, fp64=True) as ctx:
+        out = run_ops(mhd, cuda, ctx, u, b, bin_, nx, ny, nz)
+    assert bitwise_equal(out["fluidx_u"], uo)
+    assert bitwise_equal(out["advect_b"], bo)
+    assert out["calcfl"][0] == oracle64.calcfl(u, b, nx, ny, nz)
