@@ -414,52 +414,72 @@ static cudaError_t advect_x4(const AdvectArgs& a, const A4Plan& p, cudaStream_t 
     return cudaErrorInvalidValue;
 }
 
-// Warp-per-pencil marching kernel (FP32, the x sweep with the side array,
-// b(1) read in place; several boxes when their side arrays are contiguous):
-// pencils of n = 32 C cells (C = 2, 3, 4, 8), J pencils per CTA (2, or 4 by
-// advect.J), K planes per CTA (the largest that gives >= 4 waves, or
-// advect.K).  The planner's choice for pencils of 96, 128 and 256 cells (at
-// 256^3 it measured 134 against 184 us for the marching kernel), and by
-// advect.kernel = 6 for 64.
+// Warp-per-pencil marching kernel (FP32, the x sweep with the side array, b(1)
+// read in place; several boxes when their side arrays are contiguous): pencils of
+// n = C T cells, T = 32 lanes of C = 2, 3, 4, 6 or 8 cells, or T = 16 of 2 (32 cells),
+// J pencils per CTA (2, or 4 by advect.J), K planes per CTA (advect.K, or see
+// a6_planes).  The planner's choice for these lengths: at 256^3 it measured 134
+// against 184 us for the marching kernel; plain steps of 64^3 take 81 against 95 us,
+// of 32^3 53 against 58, of 192^3 1.08 against 1.52 ms (48^3 stays with k_advect2:
+// 57 against 65 us).
 struct A6Plan {
-    int C, J, K;
+    int C, J, K, T;
 };
+
+// Planes per CTA: the divisor K of nz up to 64 with the least waves x (K + 1.5), a
+// wave being the CTAs that fit at once (by registers: 10, 8, 6, 5, 5 per SM for C = 2,
+// 3, 4, 6, 8) and 1.5 planes what a CTA spends on two plane loads and a B row before
+// its first plane.  Measured per launch (K = 1, 2, 4, 8, 16, 32): 64^3 11, 9.7, 10.7, 14;
+// 96^3 18.5, 16.9, 15.1, 17; 128^3 36, 29, 25.9, 26.1; 192^3 103, 79, 66, 60, 64;
+// 256^3 -, -, -, 119, 116, 123 us: the rule takes the best of each.
+static int a6_planes(int C, int ny, int nz, int J, int boxes)
+{
+    const int per_sm = (J > 2) ? 3 : (C == 2 ? 10 : (C == 3 ? 8 : (C == 4 ? 6 : 5)));
+    const long long wave = 152LL * per_sm;
+    int K = 1;
+    long long best = -1;
+    for (int k = 1; k <= nz && k <= 64; k++) {
+        if (nz % k != 0)
+            continue;
+        const long long ctas = (long long)(ny / J) * (nz / k) * boxes;
+        const long long cost = (ctas + wave - 1) / wave * (2 * k + 3);
+        if (best < 0 || cost < best) {
+            best = cost;
+            K = k;
+        }
+    }
+    return K;
+}
 
 static bool plan_advect6(const AdvectArgs& a, bool aligned, A6Plan& p)
 {
     const int kn = tune_value(TUNE_ADVECT_KERNEL);
-    if (!kV2 || !aligned || a.axis != 0 || !(kn == 6 || (kn == 0 && (a.nx == 96 || a.nx == 128 || a.nx == 256))))
+    if (!kV2 || !aligned || a.axis != 0 || !(kn == 6 || kn == 0))
         return false;
     // several boxes: their side arrays one after the other (one tensor map covers them)
     const bool boxes_ok = a.bs.count == 1 || a.bs.w == (size_t)a.nx * a.ny * a.nz * 8;
     if (a.w == nullptr || (reinterpret_cast<uintptr_t>(a.w) & 15) != 0 || a.b1_src != a.ub || !boxes_ok)
         return false;
-    if (a.nx % 32 != 0 || !(a.nx / 32 == 2 || a.nx / 32 == 3 || a.nx / 32 == 4 || a.nx / 32 == 8))
+    p.T = (a.nx == 32) ? 16 : 32;
+    p.C = a.nx / p.T;
+    if (a.nx % p.T != 0 || !(p.C == 2 || p.C == 3 || p.C == 4 || p.C == 6 || p.C == 8))
         return false;
-    p.C = a.nx / 32;
     const int jt = tune_value(TUNE_ADVECT_J);
-    p.J = (jt == 4) ? 4 : 2;  // two pencils per CTA measured best at 256^3 (134 against 150 us)
+    p.J = (jt == 4 && p.T == 32 && p.C != 6) ? 4 : 2;  // two pencils per CTA measured best at 256^3 (134 against 150 us)
     if (a.ny % p.J != 0)
         return false;
-    const int ctas = advect6_min_ctas(p.J);
     const int kt = tune_value(TUNE_ADVECT_K);
-    p.K = 0;
-    for (int k = 1; k <= a.nz && k <= 64; k++) {
-        if (a.nz % k != 0)
-            continue;
-        if (kt ? (k == kt) : ((long long)(a.ny / p.J) * (a.nz / k) * a.bs.count >= 4LL * ctas * 152 || k == 1))
-            p.K = k;
-    }
+    p.K = (kt > 0 && kt <= 64) ? (a.nz % kt == 0 ? kt : 0) : a6_planes(p.C, a.ny, a.nz, p.J, a.bs.count);
     return p.K != 0;
 }
 
-template <int C, int J>
+template <int C, int J, int T = 32>
 static cudaError_t launch_ad6(const AdvectArgs& a, int K, cudaStream_t s)
 {
     // swizzled side-array rows (one box) for 8 and 4 cells per lane
     constexpr bool SW = (C == 8 || C == 4);
     static bool attr = false;
-    cudaError_t e = allow_smem(k_advect6<EX, C, J, SW>, attr, true);
+    cudaError_t e = allow_smem(k_advect6<EX, C, J, SW, T>, attr, true);
     if (e != cudaSuccess)
         return e;
     AdvectArgs b = a;
@@ -477,14 +497,17 @@ static cudaError_t launch_ad6(const AdvectArgs& a, int K, cudaStream_t s)
             return e;
     }
     dim3 grid(a.ny / J, (a.kcount ? a.kcount : a.nz) / K, a.bs.count);
-    return launch_after(k_advect6<EX, C, J, SW>, grid, advect6_threads(J), advect6_smem_bytes(C * 32, J), s, b, wmap);
+    return launch_after(k_advect6<EX, C, J, SW, T>, grid, advect6_threads(J), advect6_smem_bytes(C * T, J), s, b, wmap);
 }
 
 static cudaError_t advect_x6(const AdvectArgs& a, const A6Plan& p, cudaStream_t s)
 {
+    if (p.T == 16)
+        return launch_ad6<2, 2, 16>(a, p.K, s);
     switch (p.C * 10 + p.J) {
     case 82: return launch_ad6<8, 2>(a, p.K, s);
     case 84: return launch_ad6<8, 4>(a, p.K, s);
+    case 62: return launch_ad6<6, 2>(a, p.K, s);
     case 42: return launch_ad6<4, 2>(a, p.K, s);
     case 44: return launch_ad6<4, 4>(a, p.K, s);
     case 32: return launch_ad6<3, 2>(a, p.K, s);
@@ -825,14 +848,17 @@ static int multi_fluidx_parts(int n)
     return T ? (n / (kMultiFxThreads / T)) * n : 0;
 }
 
-// the advectbyzx CTA's planes along k for a class of `count` boxes of edge n
-// (the rule of plan_advect6: the largest K <= 64 that still gives 4 waves)
+// the advectbyzx CTA's planes along k for a class of `count` boxes of edge n: the
+// largest K <= 64 that leaves the class kMultiAdCtas CTAs.  The classes of a launch fill
+// its waves together, so a class needs no waves of its own and a larger K saves the
+// CTAs' prologues (24 boxes, five steps: 12.67 ms with 3040 CTAs per class, 11.56
+// with 1000, 11.35 with 500, 11.36 with 250).
+constexpr long long kMultiAdCtas = 500;
 static int multi_advect_k(int n, int count)
 {
-    const int ctas = advect6_min_ctas(kMultiAdJ);
     int K = 1;
     for (int k = 1; k <= n && k <= 64; k++)
-        if (n % k == 0 && (long long)(n / kMultiAdJ) * (n / k) * count >= 4LL * ctas * 152)
+        if (n % k == 0 && (long long)(n / kMultiAdJ) * (n / k) * count >= kMultiAdCtas)
             K = k;
     return K;
 }

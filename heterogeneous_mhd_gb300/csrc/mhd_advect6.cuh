@@ -265,12 +265,12 @@ __device__ __forceinline__ void advect6_body(AdvectArgs a, const CUtensorMap& wm
     }
 }
 
-template <bool EX, int C, int J, bool SW = false>
+template <bool EX, int C, int J, bool SW = false, int T = 32>
 __global__ void __launch_bounds__((J + 1) * 32, advect6_min_ctas(J))
     k_advect6(AdvectArgs a, const __grid_constant__ CUtensorMap wmap)
 {
     after_previous();
-    advect6_body<EX, C, J, SW, 32>(a, wmap, HwBlock{});
+    advect6_body<EX, C, J, SW, T>(a, wmap, HwBlock{});
 }
 
 }  // namespace mhd
