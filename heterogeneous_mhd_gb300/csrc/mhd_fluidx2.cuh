@@ -575,8 +575,11 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
     }
 }
 
+// Sweeps along y and z: three CTAs of 256 threads per SM for 256 cells (80 registers, as
+// the 64 KB of shared memory allow), six of 128 for 128 cells (without the bound 128
+// registers and four: 34.4 against 31.1 us per launch at 128^3).
 template <typename R, bool EX, int C, int T, int AX = 0>
-__global__ void __launch_bounds__(AX ? kSweepP * T : 256, AX ? (T <= 64 ? 3 : 1) : 0)
+__global__ void __launch_bounds__(AX ? kSweepP * T : 256, AX ? (T == 32 ? 6 : (T <= 64 ? 3 : 1)) : 0)
     k_fluidx2(FluidxArgs a, const __grid_constant__ SweepMaps tm)
 {
     after_previous();
