@@ -294,3 +294,22 @@ def test_tcgen05_conv_matches_mma_sync(kind, clos, cuda):
     assert np.array_equal(outs[0][0], outs[2][0])
     if kind != "dgrad":
         assert np.array_equal(outs[0][1], outs[2][1])
+
+
+@pytest.mark.parametrize("nb,n", [(2, 32), (3, 24)])
+def test_wgrad_more_sets_than_ctas_vs_oracle(nb, n, clos, cuda):
+    """256 and 162 tiles: CTAs that work off one and two partial sets through the two tile
+    buffers.  FP32 sums of BF16 products: 1e-4 of the gradient's norm."""
+    torch = cuda
+    rng = np.random.default_rng(n)
+    L, s = clos.cl(), clos.stream_ptr()
+    a, dz = to_bf16(torch, rng.normal(size=(nb, n, n, n, 32))), to_bf16(torch, rng.normal(size=(nb, n, n, n, 32)))
+    scr = torch.empty(int(L.mhd_cl_wgrad_scratch(clos.WG_HID, nb, n)) // 4 + 1, dtype=torch.float32, device="cuda")
+    dw = torch.zeros(32 * 27 * 32, dtype=torch.float32, device="cuda")
+    assert L.mhd_cl_wgrad(clos.WG_HID, a.data_ptr(), dz.data_ptr(), scr.data_ptr(), dw.data_ptr(), nb, n, s) == 0
+    av, zv = bf_np(a), bf_np(dz)
+    ref = np.zeros((32, 27, 32))
+    for t in range(27):
+        sh = (1 - t // 9, 1 - (t // 3) % 3, 1 - t % 3)
+        ref[:, t] = zv.reshape(-1, 32).T @ np.roll(av, sh, (1, 2, 3)).reshape(-1, 32)
+    assert rel(dw.cpu().numpy().reshape(32, 27, 32), ref) < 1e-4

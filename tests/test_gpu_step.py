@@ -288,3 +288,17 @@ def test_warp_pencil_advect_step_exact(shape, knobs, mhd, cuda, oracle32):
         autotune.apply({})
     assert bitwise_equal(u, ref[0]) and bitwise_equal(b, ref[1])
     assert bitwise_equal(uf, fast_default[0]) and bitwise_equal(bf, fast_default[1])
+
+
+@pytest.mark.parametrize("shape", [(32, 16, 16), (64, 24, 24), (96, 20, 20), (192, 16, 16), (192, 50, 50), (256, 6, 6)])
+def test_planned_warp_pencil_lengths_vs_oracle(shape, mhd, cuda, oracle32):
+    """The planner's warp-per-pencil lengths and planes per CTA, with no knob set: EXACT
+    steps bit for bit against the oracle, FAST within the step tolerance."""
+    u0, b0 = mhd.init_vortex(*shape, seed=13)
+    ref = oracle32.strang(u0, b0, *shape, 2)
+    u, b, t = run(mhd, u0, b0, shape, 2, exact=True)
+    assert bitwise_equal(u, ref[0]) and bitwise_equal(b, ref[1])
+    assert np.float32(t) == np.float32(ref[2])
+    u, b, _ = run(mhd, u0, b0, shape, 1)
+    ref = oracle32.strang(u0, b0, *shape, 1)
+    assert max(rel_l2_fields(u, b, ref[0], ref[1]).values()) <= STEP1_TOL
