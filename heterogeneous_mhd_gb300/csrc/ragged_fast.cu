@@ -62,8 +62,9 @@ cudaError_t fluidx_ragged(const FluidxArgs& in, bool exact, cudaStream_t s)
 }
 
 // J pencils per CTA: five groups of 32 lanes or ten of 16 (the group of the
-// halo pencil is the price of a small J).  K planes: as many as leave every
-// SM a few CTAs, since a CTA computes one B row before its first plane.
+// halo pencil is the price of a small J).  K planes: the K with the least waves of
+// CTAs x (K + 1.5), as a6_planes (four
+// steps of 100 x 72 x 72: 0.93 ms, 1.03 with the most planes that left 608 CTAs).
 cudaError_t advect_ragged(const AdvectArgs& in, bool exact, cudaStream_t s)
 {
     AdvectArgs a = in;
@@ -79,10 +80,16 @@ cudaError_t advect_ragged(const AdvectArgs& in, bool exact, cudaStream_t s)
         jmax = jt;
     const int nj = (a.ny + jmax - 1) / jmax;
     a.P = (a.ny + nj - 1) / nj;
-    a.K = 1;
-    for (int k = 2; k <= 32 && k <= a.nz; k++)
-        if (kt ? (k == kt) : (long long)nj * ((a.nz + k - 1) / k) * a.bs.count >= 4LL * 152)
+    const int nt = ((a.P + 1) * sh.G + 31) / 32 * 32;
+    const long long wave = 152LL * (65536 / (nt * 112) > 0 ? 65536 / (nt * 112) : 1);  // at 97-120 registers
+    long long best = -1;
+    for (int k = 1; k <= 32 && k <= a.nz; k++) {
+        const long long cost = ((long long)nj * ((a.nz + k - 1) / k) * a.bs.count + wave - 1) / wave * (2 * k + 3);
+        if (kt ? (k == 1 || k == kt) : (best < 0 || cost < best)) {
+            best = cost;
             a.K = k;
+        }
+    }
     return exact ? advect_rag_exact(a, sh, pb, wu, s) : advect_rag_fast(a, sh, pb, wu, s);
 }
 
