@@ -645,8 +645,6 @@ __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, i
     issue(k0 + 1);
     issue(k0 + 2);
     for (int k = k0; k < k1; k++) {
-        if (k + 1 == k1)
-            before_next();
         float* const fax = FAx + (k & 1) * (J + 1) * SF;
         float FA[C], bA[C], FBn[C], b3n[C], rc[C], mc[C], bb[3 * C];
         rag_tvdb_row<EX, C, D>(g, vA, b2c, dt, seam, FA, bA);
@@ -669,6 +667,8 @@ __global__ void __launch_bounds__(512) k_advect_rag(AdvectArgs a, RagShape sh, i
             face(rl, ml, rc, mc, vA);
             rag_tvdb_row<EX, C, D>(g, vB, b3, dt, seam, FBn, b3n);
         }
+        if (k + 1 == k1)
+            before_next();
         if (owner) {
             float fa1[C];
             rag_lds<C, C>(fax + (w + 1) * SF + i0, fa1);
