@@ -145,10 +145,8 @@ enum Epi { EPI_GELU = 0, EPI_LINEAR_F32 = 1, EPI_DGRAD = 2 };
 
 // y(v, co) = sum_{tap, ci} x(v + off(tap), ci) W(co, tap, ci); W is [COUT][KS^3][CIN] bf16.
 template <int CIN, int COUT, int KS, int EPI>
-__global__ void __launch_bounds__(128) k_conv(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                              const float* __restrict__ bias, void* __restrict__ y,
-                                              bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n,
-                                              long long ntiles)
+__global__ void __launch_bounds__(128) k_conv(const bf16* x, const bf16* w, const float* bias, void* y, bf16* zsave,
+                                              const bf16* zprev, int n, long long ntiles)
 {
     mhd::after_previous();
     using HL = Halo<KS>;
@@ -181,6 +179,29 @@ __global__ void __launch_bounds__(128) k_conv(const bf16* __restrict__ x, const 
         const TileIdx t = tile_of(tile, n);
         __syncthreads();  // previous tile's readers are done with sx
         load_rows<CIN, KS>(sx, x, t, n);
+        float bs[2 * NT];  // the lane's channels' bias, read while the rows land
+        if constexpr (EPI != EPI_DGRAD) {
+#pragma unroll
+            for (int j = 0; j < 2 * NT; j++)
+                bs[j] = bias[(j / 2) * 8 + 2 * (lane & 3) + (j & 1)];
+        }
+        const size_t box0 = (size_t)t.box * n * n * n;
+        auto voxel = [&](int i, int hr) {
+            const int r = (lane >> 2) + 8 * hr;
+            const int ty = 2 * i + (r >> 3), tx = r & 7;
+            return box0 + ((size_t)(t.z0 + tz) * n + (t.y0 + ty)) * n + (t.x0 + tx);
+        };
+        __nv_bfloat162 zp[MT][2][NT];  // and its pre-activations
+        if constexpr (EPI == EPI_DGRAD) {
+#pragma unroll
+            for (int i = 0; i < MT; i++)
+#pragma unroll
+                for (int hr = 0; hr < 2; hr++)
+#pragma unroll
+                    for (int j = 0; j < NT; j++)
+                        zp[i][hr][j] = *reinterpret_cast<const __nv_bfloat162*>(zprev + voxel(i, hr) * COUT + j * 8 +
+                                                                                2 * (lane & 3));
+        }
         cp_async_wait_all();
         __syncthreads();
 
@@ -229,32 +250,28 @@ __global__ void __launch_bounds__(128) k_conv(const bf16* __restrict__ x, const 
         }
 
         // epilogue: rows lane/4 and lane/4 + 8 of each m-tile, channel pair 2*(lane%4)
-        const size_t box0 = (size_t)t.box * n * n * n;
 #pragma unroll
         for (int i = 0; i < MT; i++)
 #pragma unroll
             for (int hr = 0; hr < 2; hr++) {
-                const int r = (lane >> 2) + 8 * hr;
-                const int ty = 2 * i + (r >> 3), tx = r & 7;
-                const size_t v = box0 + ((size_t)(t.z0 + tz) * n + (t.y0 + ty)) * n + (t.x0 + tx);
+                const size_t v = voxel(i, hr);
 #pragma unroll
                 for (int j = 0; j < NT; j++) {
                     const int co = j * 8 + 2 * (lane & 3);
                     float v0 = acc[i][j][2 * hr], v1 = acc[i][j][2 * hr + 1];
                     if constexpr (EPI == EPI_GELU) {
-                        const __nv_bfloat162 z = __floats2bfloat162_rn(v0 + bias[co], v1 + bias[co + 1]);
+                        const __nv_bfloat162 z = __floats2bfloat162_rn(v0 + bs[2 * j], v1 + bs[2 * j + 1]);
                         *reinterpret_cast<__nv_bfloat162*>(zsave + v * COUT + co) = z;
                         const float2 zf = __bfloat1622float2(z);
                         *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(y) + v * COUT + co) =
                             __floats2bfloat162_rn(gelu(zf.x), gelu(zf.y));
                     } else if constexpr (EPI == EPI_LINEAR_F32) {
                         *reinterpret_cast<float2*>(static_cast<float*>(y) + v * COUT + co) =
-                            make_float2(v0 + bias[co], v1 + bias[co + 1]);
+                            make_float2(v0 + bs[2 * j], v1 + bs[2 * j + 1]);
                     } else {
-                        const float2 zp =
-                            __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(zprev + v * COUT + co));
+                        const float2 z = __bfloat1622float2(zp[i][hr][j]);
                         *reinterpret_cast<__nv_bfloat162*>(static_cast<bf16*>(y) + v * COUT + co) =
-                            __floats2bfloat162_rn(v0 * gelu_grad(zp.x), v1 * gelu_grad(zp.y));
+                            __floats2bfloat162_rn(v0 * gelu_grad(z.x), v1 * gelu_grad(z.y));
                     }
                 }
             }
@@ -338,9 +355,8 @@ __device__ __forceinline__ void tc_issue_tile(uint32_t tmem, uint64_t a_desc0, u
 // in BF16 (and the pre-activation for the backward pass), or times GELU' of
 // the previous layer's pre-activation (the data gradient).
 template <int COUT, int EPI>
-__device__ __forceinline__ void tc_epilogue_row(const uint32_t (&r)[32], size_t v, const float* __restrict__ bias,
-                                                void* __restrict__ y, bf16* __restrict__ zsave,
-                                                const bf16* __restrict__ zprev)
+__device__ __forceinline__ void tc_epilogue_row(const uint32_t (&r)[32], size_t v, const float* bias,
+                                                void* y, bf16* zsave, const bf16* zprev)
 {
     __align__(16) bf16 o1[COUT];
     __align__(16) bf16 o2[COUT];
@@ -375,9 +391,8 @@ __device__ __forceinline__ void tc_epilogue_row(const uint32_t (&r)[32], size_t 
 // FP32 gelu'), which hold exactly what gelu() and gelu_grad() give on those
 // 65536 inputs: the results are the computed epilogue's bit for bit.
 template <int COUT, int EPI>
-__device__ __forceinline__ void tc_epilogue_row_tab(const uint32_t (&r)[32], size_t v, const float* __restrict__ bias,
-                                                    void* __restrict__ y, bf16* __restrict__ zsave,
-                                                    const uint4 (&zp)[COUT / 8],
+__device__ __forceinline__ void tc_epilogue_row_tab(const uint32_t (&r)[32], size_t v, const float (&bias)[COUT],
+                                                    void* y, bf16* zsave, const uint4 (&zp)[COUT / 8],
                                                     const unsigned short* __restrict__ gelu_tab,
                                                     const float* __restrict__ grad_tab)
 {
@@ -439,10 +454,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
 }
 
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(256, 1) k_conv_tc(const bf16* __restrict__ x, const bf16* __restrict__ w,
-                                                     const float* __restrict__ bias, void* __restrict__ y,
-                                                     bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n,
-                                                     long long ntiles, int* err)
+__global__ void __launch_bounds__(256, 1) k_conv_tc(const bf16* x, const bf16* w, const float* bias, void* y,
+                                                     bf16* zsave, const bf16* zprev, int n, long long ntiles,
+                                                     int* err)
 {
     mhd::after_previous();
     static_assert(COUT == 32, "one tile's accumulators are 2 x 32 TMEM columns");
@@ -596,9 +610,8 @@ __device__ __forceinline__ void mbar_arrive1(uint64_t* bar)
 
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(kTc2Warps * 32, 1)
-    k_conv_tc2(const bf16* __restrict__ x, const bf16* __restrict__ w, const float* __restrict__ bias,
-               void* __restrict__ y, bf16* __restrict__ zsave, const bf16* __restrict__ zprev, int n, long long ntiles,
-               int* err, const unsigned short* __restrict__ gelu_tab, const float* __restrict__ grad_tab)
+    k_conv_tc2(const bf16* x, const bf16* w, const float* bias, void* y, bf16* zsave, const bf16* zprev, int n,
+               long long ntiles, int* err, const unsigned short* __restrict__ gelu_tab, const float* __restrict__ grad_tab)
 {
     mhd::after_previous();
     static_assert(COUT == 32, "one tile's accumulators are 2 x 32 TMEM columns");
@@ -707,16 +720,22 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
             coords((long long)blockIdx.x + i * gridDim.x, box, z0, y0, x0);
             const int m = q * 32 + lane, vx = m >> 3, vy = m & 7;
             const size_t v = (((size_t)box * n + z0) * n + (y0 + vy)) * n + (x0 + vx);
-            // the previous layer's pre-activations of both rows, in 16-byte pieces, while the
-            // tile's MMAs run
+            // the previous layer's pre-activations of both rows, in 16-byte pieces, or the bias, while
+            // the tile's MMAs run
             uint4 zp0[COUT / 8], zp1[COUT / 8];
+            float bv[COUT];
+            if constexpr (EPI == EPI_GELU) {
+#pragma unroll
+                for (int c = 0; c < COUT; c++)
+                    bv[c] = bias[c];
+            }
             if constexpr (EPI == EPI_DGRAD) {
                 const uint4* s0 = reinterpret_cast<const uint4*>(zprev + v * COUT);
                 const uint4* s1 = reinterpret_cast<const uint4*>(zprev + (v + (size_t)n * n) * COUT);
 #pragma unroll
                 for (int c = 0; c < COUT / 8; c++) {
-                    zp0[c] = __ldg(s0 + c);
-                    zp1[c] = __ldg(s1 + c);
+                    zp0[c] = s0[c];
+                    zp1[c] = s1[c];
                 }
             }
             if (!mhd::mbar_wait_bounded(&t_full[st], (uint32_t)((i / NT) & 1), err))
@@ -729,8 +748,8 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
             __syncwarp();
             if (lane == 0)
                 mbar_arrive1(&t_empty[st]);
-            tc_epilogue_row_tab<COUT, EPI>(r0, v, bias, y, zsave, zp0, gelu_tab, grad_tab);
-            tc_epilogue_row_tab<COUT, EPI>(r1, v + (size_t)n * n, bias, y, zsave, zp1, gelu_tab, grad_tab);
+            tc_epilogue_row_tab<COUT, EPI>(r0, v, bv, y, zsave, zp0, gelu_tab, grad_tab);
+            tc_epilogue_row_tab<COUT, EPI>(r1, v + (size_t)n * n, bv, y, zsave, zp1, gelu_tab, grad_tab);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -758,8 +777,7 @@ struct WgradShape {
 
 template <int CIN, int COUTP, int KS>
 __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
-    k_wgrad(const bf16* __restrict__ a, const bf16* __restrict__ dz, float* __restrict__ part, int n,
-            long long ntiles, int nsets)
+    k_wgrad(const bf16* a, const bf16* dz, float* part, int n, long long ntiles, int nsets)
 {
     mhd::after_previous();
     using S = WgradShape<CIN, COUTP, KS>;
@@ -882,8 +900,8 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUTP, KS>::THREADS)
 constexpr int kSumWarps = 8;
 
 // out[e] = sum_p part[p * stride + e], e < len; launched on (len + 31) / 32 CTAs of kSumWarps warps
-__global__ void __launch_bounds__(kSumWarps * 32) k_sum_parts(const float* __restrict__ part, int nparts,
-                                                             size_t stride, size_t len, float* __restrict__ out)
+__global__ void __launch_bounds__(kSumWarps * 32) k_sum_parts(const float* part, int nparts, size_t stride, size_t len,
+                                                             float* out)
 {
     mhd::after_previous();
     __shared__ float red[kSumWarps][32];
@@ -908,8 +926,8 @@ __global__ void __launch_bounds__(kSumWarps * 32) k_sum_parts(const float* __res
 // layout dw[co][tap][ci] for co < cor, ci < cir, in the order of k_sum_parts
 // (a coalesced 128-byte row per partial and warp)
 constexpr int kWsumWarps = kSumWarps;
-__global__ void __launch_bounds__(kWsumWarps * 32) k_wsum(const float* __restrict__ part, int nparts, int taps,
-                                                         int cop, int cip, int cor, int cir, float* __restrict__ dw)
+__global__ void __launch_bounds__(kWsumWarps * 32) k_wsum(const float* part, int nparts, int taps, int cop, int cip,
+                                                         int cor, int cir, float* dw)
 {
     mhd::after_previous();
     __shared__ float red[kWsumWarps][32];
@@ -945,8 +963,7 @@ __global__ void __launch_bounds__(kWsumWarps * 32) k_wsum(const float* __restric
 // partials part[block][C].  Thread t reads 16-byte chunks (8 channels) of
 // chunk column t % (C/8), four rows per iteration in flight; lanes of the
 // same chunk column are summed by shuffles, then the warps in warp order.
-__global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ x, int C, size_t count,
-                                                float* __restrict__ part)
+__global__ void __launch_bounds__(256) k_colsum(const bf16* x, int C, size_t count, float* part)
 {
     mhd::after_previous();
     __shared__ float red[8][32];
@@ -966,15 +983,15 @@ __global__ void __launch_bounds__(256) k_colsum(const bf16* __restrict__ x, int 
     const uint4* x4 = reinterpret_cast<const uint4*>(x);
     size_t v = blockIdx.x * (size_t)rows + r0;
     for (; v + 3 * stride < count; v += 4 * stride) {
-        const uint4 a0 = __ldg(x4 + v * Q + q), a1 = __ldg(x4 + (v + stride) * Q + q);
-        const uint4 a2 = __ldg(x4 + (v + 2 * stride) * Q + q), a3 = __ldg(x4 + (v + 3 * stride) * Q + q);
+        const uint4 a0 = x4[v * Q + q], a1 = x4[(v + stride) * Q + q];
+        const uint4 a2 = x4[(v + 2 * stride) * Q + q], a3 = x4[(v + 3 * stride) * Q + q];
         add(a0);
         add(a1);
         add(a2);
         add(a3);
     }
     for (; v < count; v += stride)
-        add(__ldg(x4 + v * Q + q));
+        add(x4[v * Q + q]);
     // lanes l and l ^ o (o >= Q) hold the same chunk column
 #pragma unroll
     for (int k = 0; k < 8; k++)
@@ -1003,8 +1020,8 @@ __device__ __forceinline__ size_t vidx(int box, int k, int j, int i, int n)
 }
 
 // rf -> dout[0..4], rb = curl(E) - tb -> rb_out, per-block loss partials
-__global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ tgt, bf16* __restrict__ dout,
-                        float* __restrict__ rb_out, float* __restrict__ lpart, int nb, int n, float gscale)
+__global__ void k_loss1(const float* out, const bf16* tgt, bf16* dout, float* rb_out, float* lpart, int nb, int n,
+                        float gscale)
 {
     mhd::after_previous();
     __shared__ float red[32];
@@ -1029,9 +1046,6 @@ __global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ 
 #pragma unroll
         for (int c = 5; c < 16; c++)
             d[c] = __float2bfloat16_rn(0.f);
-        uint4* d4 = reinterpret_cast<uint4*>(dout + v * 16);
-        d4[0] = reinterpret_cast<const uint4*>(d)[0];
-        d4[1] = reinterpret_cast<const uint4*>(d)[1];
         const float* oi = out + vidx(box, k, j, i + 1 == n ? 0 : i + 1, n) * 8;
         const float* oj = out + vidx(box, k, j + 1 == n ? 0 : j + 1, i, n) * 8;
         const float* ok = out + vidx(box, k + 1 == n ? 0 : k + 1, j, i, n) * 8;
@@ -1042,6 +1056,9 @@ __global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ 
         const float rx = dbx - __bfloat162float(tg[5]), ry = dby - __bfloat162float(tg[6]),
                     rz = dbz - __bfloat162float(tg[7]);
         ls += rx * rx + ry * ry + rz * rz;
+        uint4* d4 = reinterpret_cast<uint4*>(dout + v * 16);
+        d4[0] = reinterpret_cast<const uint4*>(d)[0];
+        d4[1] = reinterpret_cast<const uint4*>(d)[1];
         rb_out[v * 3] = rx;
         rb_out[v * 3 + 1] = ry;
         rb_out[v * 3 + 2] = rz;
@@ -1059,7 +1076,7 @@ __global__ void k_loss1(const float* __restrict__ out, const bf16* __restrict__ 
 }
 
 // dout[5..7] = gscale * curl^T(rb)
-__global__ void k_loss2(const float* __restrict__ rb, bf16* __restrict__ dout, int nb, int n, float gscale)
+__global__ void k_loss2(const float* rb, bf16* dout, int nb, int n, float gscale)
 {
     mhd::after_previous();
     const size_t nv = (size_t)nb * n * n * n;
@@ -1084,9 +1101,8 @@ __global__ void k_loss2(const float* __restrict__ rb, bf16* __restrict__ dout, i
 
 // raw features (rho, mx, my, mz, E, Bx, By, Bz cell-centred) of one box;
 // optional FP32 copy and optional standardised BF16 rows of 16 channels
-__global__ void k_features(const float* __restrict__ u, const float* __restrict__ b, int n,
-                           const float* __restrict__ mean, const float* __restrict__ inv_std,
-                           float* __restrict__ raw, bf16* __restrict__ xo)
+__global__ void k_features(const float* u, const float* b, int n, const float* mean, const float* inv_std, float* raw,
+                           bf16* xo)
 {
     mhd::after_previous();
     const size_t nv = (size_t)n * n * n;
@@ -1099,10 +1115,6 @@ __global__ void k_features(const float* __restrict__ u, const float* __restrict_
         f[5] = 0.5f * (b[v * 3] + b[vidx(0, k, j, i + 1 == n ? 0 : i + 1, n) * 3]);
         f[6] = 0.5f * (b[v * 3 + 1] + b[vidx(0, k, j + 1 == n ? 0 : j + 1, i, n) * 3 + 1]);
         f[7] = 0.5f * (b[v * 3 + 2] + b[vidx(0, k + 1 == n ? 0 : k + 1, j, i, n) * 3 + 2]);
-        if (raw)
-#pragma unroll
-            for (int c = 0; c < 8; c++)
-                raw[v * 8 + c] = f[c];
         if (xo) {
             __align__(16) bf16 row[16];
 #pragma unroll
@@ -1115,6 +1127,10 @@ __global__ void k_features(const float* __restrict__ u, const float* __restrict_
             d[0] = reinterpret_cast<const uint4*>(row)[0];
             d[1] = reinterpret_cast<const uint4*>(row)[1];
         }
+        if (raw)
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                raw[v * 8 + c] = f[c];
     }
 }
 
@@ -1234,8 +1250,7 @@ __device__ __forceinline__ void block_add(const double (&s)[N], double* dst)
 
 // esum[2 + c] += sum over the box of out[.][c], c < 5 (the fluid corrections' means are removed,
 // so the correction conserves mass, momentum and energy as the filtered fine step does)
-__global__ void k_apply0(const float* __restrict__ out, size_t nv, double* __restrict__ esum,
-                         const float* __restrict__ dt, float dt_min)
+__global__ void k_apply0(const float* out, size_t nv, double* esum, const float* dt, float dt_min)
 {
     mhd::after_previous();
     if (skip_step(dt, dt_min))
@@ -1251,20 +1266,21 @@ __global__ void k_apply0(const float* __restrict__ out, size_t nv, double* __res
 // candidate = state + alpha * correction (fluid part with its box mean removed) into (ut, bt);
 // esum[0] += sum E, esum[1] += sum E of the candidate.  Nothing to do once an earlier attempt was
 // committed (flags[1]).
-__global__ void k_apply1(const float* __restrict__ u, const float* __restrict__ b, const float* __restrict__ out,
-                         int n, const float* __restrict__ oscale, float bscale, float alpha, float* __restrict__ ut,
-                         float* __restrict__ bt, double* __restrict__ esum, const int* __restrict__ flags,
-                         const float* __restrict__ dt, float dt_min)
+__global__ void k_apply1(const float* u, const float* b, const float* out, int n, const float* oscale, float bscale,
+                         float alpha, float* ut, float* bt, double* esum, const int* flags, const float* dt,
+                         float dt_min)
 {
     mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
         return;
     const size_t nv = (size_t)n * n * n;
     bscale *= alpha;
-    float mean[5];
+    float mean[5], os[5];
 #pragma unroll
-    for (int q = 0; q < 5; q++)
+    for (int q = 0; q < 5; q++) {
         mean[q] = (float)(esum[2 + q] / (double)nv);
+        os[q] = oscale[q];
+    }
     double e0 = 0.0, e1 = 0.0;
     for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
         const int i = (int)(v % n), j = (int)((v / n) % n), k = (int)(v / ((size_t)n * n));
@@ -1272,22 +1288,32 @@ __global__ void k_apply1(const float* __restrict__ u, const float* __restrict__ 
         const float* oi = out + vidx(0, k, j, i + 1 == n ? 0 : i + 1, n) * 8;
         const float* oj = out + vidx(0, k, j + 1 == n ? 0 : j + 1, i, n) * 8;
         const float* ok = out + vidx(0, k + 1 == n ? 0 : k + 1, j, i, n) * 8;
+        // the voxel's loads before its stores (which could alias them)
+        float uc[5], bc[3];
 #pragma unroll
         for (int q = 0; q < 5; q++)
-            ut[v * 5 + q] = u[v * 5 + q] + alpha * oscale[q] * (o[q] - mean[q]);
-        bt[v * 3] = b[v * 3] + bscale * (-(oj[7] - o[7]) + (ok[6] - o[6]));
-        bt[v * 3 + 1] = b[v * 3 + 1] + bscale * (-(ok[5] - o[5]) + (oi[7] - o[7]));
-        bt[v * 3 + 2] = b[v * 3 + 2] + bscale * (-(oi[6] - o[6]) + (oj[5] - o[5]));
-        e0 += u[v * 5 + 4];
-        e1 += ut[v * 5 + 4];
+            uc[q] = u[v * 5 + q];
+        e0 += uc[4];
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+            uc[q] = uc[q] + alpha * os[q] * (o[q] - mean[q]);
+        bc[0] = b[v * 3] + bscale * (-(oj[7] - o[7]) + (ok[6] - o[6]));
+        bc[1] = b[v * 3 + 1] + bscale * (-(ok[5] - o[5]) + (oi[7] - o[7]));
+        bc[2] = b[v * 3 + 2] + bscale * (-(oi[6] - o[6]) + (oj[5] - o[5]));
+        e1 += uc[4];
+#pragma unroll
+        for (int q = 0; q < 5; q++)
+            ut[v * 5 + q] = uc[q];
+#pragma unroll
+        for (int q = 0; q < 3; q++)
+            bt[v * 3 + q] = bc[q];
     }
     const double e[2] = {e0, e1};
     block_add<2>(e, esum);
 }
 
 // positivity of the candidate (it needs the neighbours' candidate faces: a second pass)
-__global__ void k_apply2(const float* __restrict__ ut, const float* __restrict__ bt, int n, int* __restrict__ flags,
-                         const float* __restrict__ dt, float dt_min)
+__global__ void k_apply2(const float* ut, const float* bt, int n, int* flags, const float* dt, float dt_min)
 {
     mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
@@ -1311,10 +1337,8 @@ __global__ void k_apply2(const float* __restrict__ ut, const float* __restrict__
 
 // commit the candidate unless a check failed (flags[1] = 1 once committed); the last attempt
 // counts a fallback on the device when it fails too
-__global__ void k_apply3(float* __restrict__ u, float* __restrict__ b, const float* __restrict__ ut,
-                         const float* __restrict__ bt, size_t nv, int* __restrict__ flags,
-                         const double* __restrict__ esum, float ecap, long long* __restrict__ fallbacks, int last,
-                         const float* __restrict__ dt, float dt_min)
+__global__ void k_apply3(float* u, float* b, const float* ut, const float* bt, size_t nv, int* flags, const double* esum,
+                         float ecap, long long* fallbacks, int last, const float* dt, float dt_min)
 {
     mhd::after_previous();
     if (flags[1] || skip_step(dt, dt_min))
@@ -1327,34 +1351,30 @@ __global__ void k_apply3(float* __restrict__ u, float* __restrict__ b, const flo
         return;
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicExch(&flags[2], 1);  // committed: read by the next attempt's kernels as flags[1]
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nv * 5; e += (size_t)gridDim.x * blockDim.x)
-        u[e] = ut[e];
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nv * 3; e += (size_t)gridDim.x * blockDim.x)
-        b[e] = bt[e];
+    mhd::copy_strided(ut, u, nv * 5);
+    mhd::copy_strided(bt, b, nv * 3);
 }
 
 // ------------------------------------------------------------ optimiser and weight packing
 
-__global__ void k_adamw(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                        float* __restrict__ v, size_t count, float lr, float b1, float b2, float eps, float wd,
-                        float c1, float c2)
+__global__ void k_adamw(float* p, const float* g, float* m, float* v, size_t count, float lr, float b1, float b2,
+                        float eps, float wd, float c1, float c2)
 {
     mhd::after_previous();
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x) {
-        const float gg = g[e];
+        const float gg = g[e], pp = p[e];
         const float mm = b1 * m[e] + (1.f - b1) * gg;
         const float vv = b2 * v[e] + (1.f - b2) * gg * gg;
         m[e] = mm;
         v[e] = vv;
         const float mh = mm / c1, vh = vv / c2;
-        p[e] = p[e] - lr * (mh / (sqrtf(vh) + eps) + wd * p[e]);
+        p[e] = pp - lr * (mh / (sqrtf(vh) + eps) + wd * pp);
     }
 }
 
 // master W[co][tap][ci] (FP32, ci < cir, co < cor) -> forward bf16 [cop][taps][cip] and
 // data-gradient bf16 [cip][taps][cop] with the taps flipped (zeros in the padding)
-__global__ void k_pack(const float* __restrict__ w, int cor, int cir, int taps, int cop, int cip,
-                       bf16* __restrict__ wf, bf16* __restrict__ wd)
+__global__ void k_pack(const float* w, int cor, int cir, int taps, int cop, int cip, bf16* wf, bf16* wd)
 {
     mhd::after_previous();
     const size_t tot = (size_t)cop * taps * cip;

@@ -178,6 +178,13 @@ __global__ void __launch_bounds__(512) k_advect2(AdvectArgs a)
             bv[m] = (comp == 1) ? bb[3 * m + 1] : bb[3 * m + 2];
             b1own[m] = bb[3 * m];
         }
+        const R* b1s = static_cast<const R*>(a.b1_src);
+        if (b1s != ub && live && r < P) {  // early: its latency passes behind the row's work
+            ldg_chunk<R, C * 3>(b1s + (pc + i0) * 3, bb);
+#pragma unroll
+            for (int m = 0; m < C; m++)
+                b1own[m] = bb[3 * m];
+        }
     }
     R bnew[C], F[C];
     tvdb_row<R, EX, C, T>(g, vr, bv, dt, seam, F, bnew);
@@ -197,14 +204,6 @@ __global__ void __launch_bounds__(512) k_advect2(AdvectArgs a)
     // ---- A1/A2/B1/B2 combine by the A-row threads of the owned pencils
     if (live && r < P) {
         const size_t cell0 = pc + i0;  // pencil (j0+r, k)
-        const R* b1s = static_cast<const R*>(a.b1_src);
-        if (b1s != ub) {
-            R bb[C * 3];
-            ldg_chunk<R, C * 3>(b1s + cell0 * 3, bb);
-#pragma unroll
-            for (int m = 0; m < C; m++)
-                b1own[m] = bb[3 * m];
-        }
         R out[C * 3];
         const R* fa1 = FXs + (size_t)(r + 1) * n + i0;
         const R* fb = FXs + (size_t)(P + 1 + r) * n + i0;

@@ -739,32 +739,35 @@ __global__ void __launch_bounds__(256) k_transpose(TransposeArgs a)
 }
 
 // copy_matrix (C/copy_matrix.c:9-38) as a vectorised device copy.
-static __global__ void __launch_bounds__(256) k_copy16(const uint4* __restrict__ src, uint4* __restrict__ dst, size_t n16)
+static __global__ void __launch_bounds__(256) k_copy16(const uint4* src, uint4* dst, size_t n16)
 {
     after_previous();
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n16; e += (size_t)gridDim.x * blockDim.x)
-        dst[e] = src[e];
+    copy_strided(src, dst, n16);
 }
 
 // u and b in one launch (a small state's copies are launch latency)
-static __global__ void __launch_bounds__(256) k_copy16x2(const uint4* __restrict__ src0, uint4* __restrict__ dst0,
-                                                         size_t n0, const uint4* __restrict__ src1,
-                                                         uint4* __restrict__ dst1, size_t n1)
+static __global__ void __launch_bounds__(256) k_copy16x2(const uint4* src0, uint4* dst0, size_t n0, const uint4* src1,
+                                                         uint4* dst1, size_t n1)
 {
     after_previous();
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n0 + n1; e += (size_t)gridDim.x * blockDim.x) {
-        if (e < n0)
-            dst0[e] = src0[e];
-        else
-            dst1[e - n0] = src1[e - n0];
+    const size_t n = n0 + n1, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += 4 * step) {
+        uint4 x[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (const size_t i = e + q * step; i < n)
+                x[q] = i < n0 ? src0[i] : src1[i - n0];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (const size_t i = e + q * step; i < n)
+                (i < n0 ? dst0 + i : dst1 + (i - n0))[0] = x[q];
     }
 }
 
-static __global__ void __launch_bounds__(256) k_copy4(const float* __restrict__ src, float* __restrict__ dst, size_t n4)
+static __global__ void __launch_bounds__(256) k_copy4(const float* src, float* dst, size_t n4)
 {
     after_previous();
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n4; e += (size_t)gridDim.x * blockDim.x)
-        dst[e] = src[e];
+    copy_strided(src, dst, n4);
 }
 
 // ------------------------------------------------------------------ calcfl
@@ -773,8 +776,8 @@ static __global__ void __launch_bounds__(256) k_copy4(const float* __restrict__ 
 // over a contiguous range of cells (blockDim cells per CTA) and the last NaN
 // index in the range (cell0 + the index in the range: the index in the box).
 template <typename R, bool EX>
-__global__ void __launch_bounds__(256) k_calcfl(const R* __restrict__ u, const R* __restrict__ b, size_t ncell,
-                                                size_t cell0, CflPart<R>* part, BoxStrides bs)
+__global__ void __launch_bounds__(256) k_calcfl(const R* u, const R* b, size_t ncell, size_t cell0, CflPart<R>* part,
+                                                BoxStrides bs)
 {
     after_previous();
     __shared__ R rm[8];
@@ -830,8 +833,7 @@ __global__ void __launch_bounds__(256) k_calcfl(const R* __restrict__ u, const R
 // NaN index (both order-free, so the result is the one-CTA reduction's).
 // One CTA reading 65536 partials is bound by its own L1 sector throughput.
 template <typename R>
-__global__ void __launch_bounds__(256) k_cfl_reduce(const CflPart<R>* __restrict__ part, int nparts,
-                                                    CflPart<R>* __restrict__ out)
+__global__ void __launch_bounds__(256) k_cfl_reduce(const CflPart<R>* part, int nparts, CflPart<R>* out)
 {
     before_next();  // a few CTAs: the next grid spreads over the other SMs
     after_previous();

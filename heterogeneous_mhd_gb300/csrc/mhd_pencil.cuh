@@ -118,27 +118,25 @@ constexpr int kSweepPad = 8;
 
 // Global chunk loads/stores of NF consecutive values with the widest vector
 // the alignment allows (the caller guarantees it: 16 B for NF % 4 == 0, 8 B
-// for NF % 2 == 0).
+// for NF % 2 == 0).  Loads: whole vectors (a plain C++ load of which some
+// components are used is split into narrow ones) on the coherent path, of data that this
+// kernel has not written; the empty volatile statement keeps them behind after_previous().
 template <typename R, int NF>
 __device__ __forceinline__ void ldg_chunk(const R* src, R (&dst)[NF])
 {
-    if constexpr (sizeof(R) == 4 && NF % 4 == 0) {
-        const float4* s4 = reinterpret_cast<const float4*>(src);
+    if constexpr (sizeof(R) == 4 && NF % 2 == 0) {
+        size_t p = __cvta_generic_to_global(src);
+        asm volatile("" : "+l"(p));
+        if constexpr (NF % 4 == 0) {
 #pragma unroll
-        for (int v = 0; v < NF / 4; v++) {
-            const float4 x = __ldg(s4 + v);
-            dst[4 * v] = x.x;
-            dst[4 * v + 1] = x.y;
-            dst[4 * v + 2] = x.z;
-            dst[4 * v + 3] = x.w;
-        }
-    } else if constexpr (sizeof(R) == 4 && NF % 2 == 0) {
-        const float2* s2 = reinterpret_cast<const float2*>(src);
+            for (int v = 0; v < NF; v += 4)
+                asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                    : "=f"(dst[v]), "=f"(dst[v + 1]), "=f"(dst[v + 2]), "=f"(dst[v + 3])
+                    : "l"(p + 4 * v));
+        } else {
 #pragma unroll
-        for (int v = 0; v < NF / 2; v++) {
-            const float2 x = __ldg(s2 + v);
-            dst[2 * v] = x.x;
-            dst[2 * v + 1] = x.y;
+            for (int v = 0; v < NF; v += 2)
+                asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(dst[v]), "=f"(dst[v + 1]) : "l"(p + 4 * v));
         }
     } else {
 #pragma unroll

@@ -34,6 +34,31 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void before_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// What a dependent kernel may read, and how: it is live while the kernels before it still
+// write, so data that another kernel writes (state, side arrays, partials, flags,
+// activations, weights, dt) is read after after_previous() through plain loads or
+// asynchronous copies.  __ldg and __restrict__ promise the compiler and the read-only path
+// that the data is constant for the kernel's lifetime; they are kept for constant tables.
+// Loops therefore load what they need before they store (a store may alias a later load).
+
+// src to dst by the whole grid, four loads in flight a thread (the compiler cannot
+// move a load above a store that may alias it).
+template <typename V>
+__device__ __forceinline__ void copy_strided(const V* src, V* dst, size_t n)
+{
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; e + 3 * step < n; e += 4 * step) {
+        const V x0 = src[e], x1 = src[e + step], x2 = src[e + 2 * step], x3 = src[e + 3 * step];
+        dst[e] = x0;
+        dst[e + step] = x1;
+        dst[e + 2 * step] = x2;
+        dst[e + 3 * step] = x3;
+    }
+    for (; e < n; e += step)
+        dst[e] = src[e];
+}
+
 // A launch that may start while the one before it in the stream drains; the
 // kernel begins with after_previous().  Captured into a graph it becomes a
 // programmatic edge.
