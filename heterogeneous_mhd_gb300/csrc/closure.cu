@@ -720,8 +720,8 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
             coords((long long)blockIdx.x + i * gridDim.x, box, z0, y0, x0);
             const int m = q * 32 + lane, vx = m >> 3, vy = m & 7;
             const size_t v = (((size_t)box * n + z0) * n + (y0 + vy)) * n + (x0 + vx);
-            // the previous layer's pre-activations of both rows, in 16-byte pieces, or the bias, while
-            // the tile's MMAs run
+            // the previous layer's pre-activations of both rows, in 16-byte pieces where they are
+            // aligned, or the bias, while the tile's MMAs run
             uint4 zp0[COUT / 8], zp1[COUT / 8];
             float bv[COUT];
             if constexpr (EPI == EPI_GELU) {
@@ -730,12 +730,21 @@ __global__ void __launch_bounds__(kTc2Warps * 32, 1)
                     bv[c] = bias[c];
             }
             if constexpr (EPI == EPI_DGRAD) {
-                const uint4* s0 = reinterpret_cast<const uint4*>(zprev + v * COUT);
-                const uint4* s1 = reinterpret_cast<const uint4*>(zprev + (v + (size_t)n * n) * COUT);
+                const bf16 *z0p = zprev + v * COUT, *z1p = zprev + (v + (size_t)n * n) * COUT;
+                if ((reinterpret_cast<uintptr_t>(zprev) & 15) == 0) {
 #pragma unroll
-                for (int c = 0; c < COUT / 8; c++) {
-                    zp0[c] = s0[c];
-                    zp1[c] = s1[c];
+                    for (int c = 0; c < COUT / 8; c++) {
+                        zp0[c] = reinterpret_cast<const uint4*>(z0p)[c];
+                        zp1[c] = reinterpret_cast<const uint4*>(z1p)[c];
+                    }
+                } else {  // a tensor that starts on a channel pair only
+                    const uint32_t *s0 = reinterpret_cast<const uint32_t*>(z0p),
+                                   *s1 = reinterpret_cast<const uint32_t*>(z1p);
+#pragma unroll
+                    for (int c = 0; c < COUT / 8; c++) {
+                        zp0[c] = make_uint4(s0[4 * c], s0[4 * c + 1], s0[4 * c + 2], s0[4 * c + 3]);
+                        zp1[c] = make_uint4(s1[4 * c], s1[4 * c + 1], s1[4 * c + 2], s1[4 * c + 3]);
+                    }
                 }
             }
             if (!mhd::mbar_wait_bounded(&t_full[st], (uint32_t)((i / NT) & 1), err))

@@ -313,3 +313,26 @@ def test_wgrad_more_sets_than_ctas_vs_oracle(nb, n, clos, cuda):
         sh = (1 - t // 9, 1 - (t // 3) % 3, 1 - t % 3)
         ref[:, t] = zv.reshape(-1, 32).T @ np.roll(av, sh, (1, 2, 3)).reshape(-1, 32)
     assert rel(dw.cpu().numpy().reshape(32, 27, 32), ref) < 1e-4
+
+
+@pytest.mark.parametrize("n", [16, 24, 32])
+def test_dgrad_pre_activations_on_a_channel_pair(n, clos, cuda):
+    """The previous layer's pre-activations may start on any channel pair (4 bytes): the same
+    bits as with an aligned tensor, in the tcgen05 kernels (16, 32) and mma.sync (24)."""
+    torch = cuda
+    L, s = clos.cl(), clos.stream_ptr()
+    rng = np.random.default_rng(n)
+    nv = n ** 3
+    dz, z, w = (to_bf16(torch, rng.normal(size=k)) for k in (nv * 32, nv * 32, 32 * 27 * 32))
+    base = torch.zeros(nv * 32 + 8, dtype=torch.bfloat16, device="cuda")
+    shifted = base[2:2 + nv * 32]
+    shifted.copy_(z)
+    assert z.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 4
+    got = []
+    for zp in (z, shifted):
+        y = torch.zeros(nv * 32, dtype=torch.bfloat16, device="cuda")
+        assert L.mhd_cl_conv(clos.DGRAD_HID, dz.data_ptr(), w.data_ptr(), None, y.data_ptr(), None, zp.data_ptr(), 1, n,
+                             s) == 0
+        got.append(bf_np(y))
+    assert clos.cl().mhd_cl_device_errors() == 0
+    assert np.array_equal(got[0], got[1]) and np.abs(got[0]).max() > 0
