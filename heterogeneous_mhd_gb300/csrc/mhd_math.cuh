@@ -450,9 +450,10 @@ __device__ __forceinline__ R tvdb_smooth(R vm, R v, R vp)
     using W = wide_t<R, EX>;
     if constexpr (EX && sizeof(R) == 4) {
         // the sum of two floats rounds alike with and without the double between, and the
-        // quarter is exact unless it is subnormal
-        const R f = vm + vp, t = r_fma(R(2), v, f);
-        return (t == R(0) || fabsf(t) > 0x1p-120f) ? t * R(0.25) : R((W(f) + W(2.0) * W(v)) / W(4.0));
+        // quarter is exact unless it is subnormal; the sum may overflow where the quarter does not
+        const R f = vm + vp, t = r_fma(R(2), v, f), m = fabsf(t);
+        return (t == R(0) || (m > 0x1p-120f && m < 0x1p127f)) ? t * R(0.25)
+                                                              : R((W(f) + W(2.0) * W(v)) / W(4.0));
     } else if constexpr (EX)  // 2 v is exact
         return r_mul(r_fma(R(2), v, vm + vp), R(0.25));
     else
