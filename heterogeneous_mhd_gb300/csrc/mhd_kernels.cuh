@@ -302,94 +302,137 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
     const int im = (i == 0) ? n - 1 : i - 1;
     const int me = lp * n + i, mep = lp * n + ip, mem = lp * n + im;
 
-    R q[5], f[3];
-#pragma unroll
-    for (int c = 0; c < 5; c++)
-        q[c] = su[5 * me + c];
-    {   // cell-centred B (C/fluidx.c:71-81): b/2 + b(neighbour face)/2
-        const R* bj = sb + 3 * lp * n;
-        const R* bjp = sb + 3 * (lp + 1) * n;
-        const R* bkp = sbk + 3 * lp * n;
-        f[0] = R(0.5) * __dadd_rn(bj[3 * i], bj[3 * ip]);
-        f[1] = R(0.5) * __dadd_rn(bj[3 * i + 1], bjp[3 * i + 1]);
-        f[2] = R(0.5) * __dadd_rn(bj[3 * i + 2], bkp[3 * i + 2]);
-    }
-
-    // Fluxes are kept undivided (2 flux, 2 dfrm, 2 dflm), the half goes into the step.
-    // ---- stage 1 (C/tvd1.c:33-49)
-    R v[5], ci, fr[5], flux[5], u1[5];
-    cell_flux64(q, f, v, ci);
-    R c = pencil_max64(ci, red, n, lp);
-    scale_flux<R, true>(v, c);
-#pragma unroll
-    for (int s = 0; s < 5; s++) {
-        fr[s] = scale64(c, __dadd_rn(q[s], v[s]));
-        if (act)
-            xa[5 * me + s] = scale64(c, __dsub_rn(q[s], v[s]));  // fl(i-1) = c*wl(i)
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < 5; s++) {
-        flux[s] = __dsub_rn(fr[s], xa[5 * mep + s]);
-        if (act)
-            xb[5 * me + s] = flux[s];
-    }
-    __syncthreads();
-    {
-        const R hdt = R(-0.25) * dt;
+    // The new q.  FEW: the forms with fewer FP64 operations, whose fluxes are kept undivided
+    // (2 flux, 2 dfrm, 2 dflm; the half goes into the step); true if a value was out of their range.
+    R q[5];
+    auto sweep = [&](auto few) -> bool {
+        constexpr bool FEW = decltype(few)::value;
+        Range64 rg;
+        R f[3];
 #pragma unroll
         for (int s = 0; s < 5; s++)
-            u1[s] = __dadd_rn(__dadd_rn(q[s], __dmul_rn(hdt, __dsub_rn(flux[s], xb[5 * mem + s]))), R(0));
-    }
+            q[s] = su[5 * me + s];
+        {   // cell-centred B (C/fluidx.c:71-81): b/2 + b(neighbour face)/2
+            const R* bj = sb + 3 * (lp * n + i);
+            const R bn[3] = {sb[3 * (lp * n + ip)], sb[3 * ((lp + 1) * n + i) + 1], sbk[3 * (lp * n + i) + 2]};
+#pragma unroll
+            for (int s = 0; s < 3; s++) {
+                if constexpr (FEW) {
+                    f[s] = R(0.5) * __dadd_rn(bj[s], bn[s]);
+                    rg.see(bj[s]);
+                    rg.see(bn[s]);
+                    rg.see(f[s]);
+                } else {
+                    f[s] = R(0.5) * bj[s] + R(0.5) * bn[s];
+                }
+            }
+        }
+        // w's fluxes: fr = c (w + v), gl = c (w - v)
+        auto fluxes = [&](const R (&w)[5], R (&fr)[5], R (&gl)[5]) {
+            R v[5], ci;
+            if constexpr (FEW) {
+                rg.see(w[4]);
+                cell_flux64(w, f, v, ci);
+            } else {
+                cell_flux<R, EX>(w, f, v, ci);
+            }
+            const R c = pencil_max64(ci, red, n, lp);
+            scale_flux<R, EX>(v, c);
+#pragma unroll
+            for (int s = 0; s < 5; s++) {
+                if constexpr (FEW) {
+                    fr[s] = __dmul_rn(c, __dadd_rn(w[s], v[s]));
+                    gl[s] = __dmul_rn(c, __dsub_rn(w[s], v[s]));
+                    rg.see(fr[s]);
+                    rg.see(gl[s]);
+                } else {
+                    fr[s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[s], R(1), v[s]));
+                    gl[s] = scale0<R, EX>(c, lin<R, EX>(R(1), w[s], R(-1), v[s]));
+                }
+            }
+        };
+        auto diff = [&](R x, R y) {  // the half of x - y, undivided in FEW
+            return FEW ? __dsub_rn(x, y) : lin<R, EX>(R(0.5), x, R(-0.5), y);
+        };
+        // w + h (flux(i) - flux(i-1)), twice the difference in FEW
+        auto advance = [&](R w, R h, R x, R y) {
+            if constexpr (FEW)
+                return __dadd_rn(__dadd_rn(w, __dmul_rn(R(0.5) * h, __dsub_rn(x, y))), R(0));
+            else
+                return lin<R, EX>(R(1), w, h, lin<R, EX>(R(1), x, R(-1), y));
+        };
 
-    // ---- stage 2 (C/tvd1.c:51-116)
-    cell_flux64(u1, f, v, ci);
-    c = pencil_max64(ci, red, n, lp);
-    scale_flux<R, true>(v, c);
-    R g[5];
+        // ---- stage 1 (C/tvd1.c:33-49)
+        R fr[5], g[5], flux[5], u1[5];
+        if constexpr (FEW)
+            rg.see(dt);
+        fluxes(q, fr, g);
 #pragma unroll
-    for (int s = 0; s < 5; s++) {
-        fr[s] = scale64(c, __dadd_rn(u1[s], v[s]));
-        g[s] = scale64(c, __dsub_rn(u1[s], v[s]));
-        if (act) {
-            xa[5 * me + s] = fr[s];
-            xa[5 * (np + me) + s] = g[s];
-        }
-    }
-    __syncthreads();
-    R gp[5];
-#pragma unroll
-    for (int s = 0; s < 5; s++) {
-        gp[s] = xa[5 * (np + mep) + s];  // fl(i) = g(i+1)
-        const R dfrm = __dsub_rn(fr[s], xa[5 * mem + s]);
-        const R dflm = __dsub_rn(g[s], gp[s]);
-        if (act) {
-            xb[5 * me + s] = dfrm;
-            xb[5 * (np + me) + s] = dflm;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < 5; s++) {
-        // dfrp(i) = dfrm(i+1), dflp(i) = dflm(i+1)
-        const R dfr = vanleer64(xb[5 * mep + s], xb[5 * me + s]);
-        const R dfl = vanleer64(xb[5 * (np + mep) + s], xb[5 * (np + me) + s]);
-        flux[s] = __dadd_rn(__dsub_rn(fr[s], gp[s]), __dsub_rn(dfr, dfl));
-        if (act)
-            xa[5 * me + s] = flux[s];
-    }
-    __syncthreads();
-    {
-        const R mdt = R(-0.5) * dt;
+        for (int s = 0; s < 5; s++)
+            if (act)
+                xa[5 * me + s] = g[s];  // fl(i-1) = c*wl(i)
+        __syncthreads();
 #pragma unroll
         for (int s = 0; s < 5; s++) {
-            const R un =
-                __dadd_rn(__dadd_rn(q[s], __dmul_rn(mdt, __dsub_rn(flux[s], xa[5 * mem + s]))), R(0));
-            q[s] = un;
+            flux[s] = diff(fr[s], xa[5 * mep + s]);
             if (act)
-                su[5 * me + s] = un;  // own slot: no other thread reads su after staging
+                xb[5 * me + s] = flux[s];
         }
-    }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < 5; s++)
+            u1[s] = advance(q[s], R(-0.5) * dt, flux[s], xb[5 * mem + s]);
+
+        // ---- stage 2 (C/tvd1.c:51-116)
+        fluxes(u1, fr, g);
+#pragma unroll
+        for (int s = 0; s < 5; s++)
+            if (act) {
+                xa[5 * me + s] = fr[s];
+                xa[5 * (np + me) + s] = g[s];
+            }
+        __syncthreads();
+        R gp[5];
+#pragma unroll
+        for (int s = 0; s < 5; s++) {
+            gp[s] = xa[5 * (np + mep) + s];  // fl(i) = g(i+1)
+            const R dfrm = diff(fr[s], xa[5 * mem + s]);
+            const R dflm = diff(g[s], gp[s]);
+            if constexpr (FEW) {
+                rg.see(dfrm);
+                rg.see(dflm);
+            }
+            if (act) {
+                xb[5 * me + s] = dfrm;
+                xb[5 * (np + me) + s] = dflm;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < 5; s++) {
+            // dfrp(i) = dfrm(i+1), dflp(i) = dflm(i+1)
+            const R a1 = xb[5 * mep + s], a0 = xb[5 * me + s];
+            const R b1 = xb[5 * (np + mep) + s], b0 = xb[5 * (np + me) + s];
+            if constexpr (FEW)
+                flux[s] = __dadd_rn(__dsub_rn(fr[s], gp[s]), __dsub_rn(vanleer64(a1, a0), vanleer64(b1, b0)));
+            else
+                flux[s] = lin<R, EX>(R(0.5), lin<R, EX>(R(1), fr[s], R(-1), gp[s]), R(0.5),
+                                     lin<R, EX>(R(1), vanleer<R, EX>(a1, a0), R(-1), vanleer<R, EX>(b1, b0)));
+            if (act)
+                xa[5 * me + s] = flux[s];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < 5; s++)
+            q[s] = advance(q[s], -dt, flux[s], xa[5 * mem + s]);
+        return !rg.ok();
+    };
+    if (__syncthreads_or(sweep(std::true_type{})))
+        sweep(std::false_type{});
+#pragma unroll
+    for (int s = 0; s < 5; s++)
+        if (act)
+            su[5 * me + s] = q[s];  // own slot: no other thread reads su after staging
 
     // ---- optional calcfl epilogue on the new state
     if (a.cfl_part) {
@@ -518,45 +561,81 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
         BV[it] = ub[(pc + i) * 3 + comp];
     }
     __syncthreads();
-    // Phase 2: 1-2-1 smoothing (C/advectbyzxA1.c:37-41), b*vg (C/tvdb.c:31-34).
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int r = it / n, i = it - r * n;
-        const int ip = (i + 1 == n) ? 0 : i + 1, im = (i == 0) ? n - 1 : i - 1;
-        const R* row = VR + r * n;
-        const R vg = tvdb_smooth<R, EX>(row[im], row[i], row[ip]);
-        VG[it] = vg;
-        T2[it] = BV[it] * vg;
-    }
-    __syncthreads();
-    // Phase 3: vh and the upwind half-step flux (C/tvdb.c:25-46).
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int r = it / n, i = it - r * n;
-        const int ip = (i + 1 == n) ? 0 : i + 1;
-        const R vh = tvdb_vh<R, EX>(VG[it], VG[r * n + ip]);
-        VH[it] = vh;
-        F1[it] = (vh > R(0)) ? T2[it] : T2[r * n + ip];
-    }
-    __syncthreads();
-    // Phase 4: half step b1 (C/tvdb.c:47-52), then vg*b1.
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int r = it / n, i = it - r * n;
-        const int im = (i == 0) ? n - 1 : i - 1;
-        R b1;
-        if constexpr (EX)
-            b1 = tvdb_half<R, EX>(BV[it], F1[it], F1[r * n + im], dt);
-        else
-            b1 = BV[it] - (F1[it] - F1[r * n + im]) * dt * R(0.5);
-        T2[it] = VG[it] * b1;
-    }
-    __syncthreads();
-    // Phase 5: limited upwind flux (C/tvdb.c:54-78).
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-        const int r = it / n, i = it - r * n;
-        const int ip = (i + 1 == n) ? 0 : i + 1;
-        const int ipp = (ip + 1 == n) ? 0 : ip + 1;
-        const int im = (i == 0) ? n - 1 : i - 1;
-        const R* vb = T2 + r * n;
-        FX[it] = tvdb_flux<R, EX>(vb[im], vb[i], vb[ip], vb[ipp], VH[it], dt);
+    // Phases 2 to 5 from VR and BV into FX.  FEW (FP64): the forms with fewer FP64
+    // operations; true if a value was out of their range.
+    auto rows = [&](auto few) -> bool {
+        constexpr bool FEW = decltype(few)::value;
+        Range64 rg;
+        // Phase 2: 1-2-1 smoothing (C/advectbyzxA1.c:37-41), b*vg (C/tvdb.c:31-34).
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int r = it / n, i = it - r * n;
+            const int ip = (i + 1 == n) ? 0 : i + 1, im = (i == 0) ? n - 1 : i - 1;
+            const R* row = VR + r * n;
+            R vg;
+            if constexpr (FEW) {  // 2 v is exact
+                vg = r_mul(r_fma(R(2), row[i], row[im] + row[ip]), R(0.25));
+                rg.see(row[i]);
+                rg.see(vg);
+                rg.see(BV[it]);
+            } else {
+                vg = tvdb_smooth<R, EX>(row[im], row[i], row[ip]);
+            }
+            VG[it] = vg;
+            T2[it] = BV[it] * vg;
+        }
+        __syncthreads();
+        // Phase 3: vh and the upwind half-step flux (C/tvdb.c:25-46).
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int r = it / n, i = it - r * n;
+            const int ip = (i + 1 == n) ? 0 : i + 1;
+            const R a0 = VG[it], a1 = VG[r * n + ip];
+            const R vh = FEW ? a0 + a1 : tvdb_vh<R, EX>(a0, a1);  // only its sign is used
+            VH[it] = vh;
+            F1[it] = (vh > R(0)) ? T2[it] : T2[r * n + ip];
+        }
+        __syncthreads();
+        // Phase 4: half step b1 (C/tvdb.c:47-52), then vg*b1.
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int r = it / n, i = it - r * n;
+            const int im = (i == 0) ? n - 1 : i - 1;
+            R b1;
+            if constexpr (FEW)
+                b1 = r_fma(R(-0.5), (F1[it] - F1[r * n + im]) * dt, BV[it]);
+            else if constexpr (EX)
+                b1 = tvdb_half<R, EX>(BV[it], F1[it], F1[r * n + im], dt);
+            else
+                b1 = BV[it] - (F1[it] - F1[r * n + im]) * dt * R(0.5);
+            const R vb = VG[it] * b1;
+            T2[it] = vb;
+            if constexpr (FEW)
+                rg.see(vb);
+        }
+        __syncthreads();
+        // Phase 5: limited upwind flux (C/tvdb.c:54-78).
+        for (int it = threadIdx.x; it < items; it += blockDim.x) {
+            const int r = it / n, i = it - r * n;
+            const int ip = (i + 1 == n) ? 0 : i + 1;
+            const int ipp = (ip + 1 == n) ? 0 : ip + 1;
+            const int im = (i == 0) ? n - 1 : i - 1;
+            const R* vb = T2 + r * n;
+            if constexpr (FEW) {  // the limiter on the undivided differences
+                const bool up = positive64(VH[it]);
+                const R w = up ? vb[i] : vb[ip];
+                const R dp = vb[ip] - (up ? vb[i] : vb[ipp]), dm = vb[i] - (up ? vb[im] : vb[ip]);
+                rg.see(dp);
+                rg.see(dm);
+                FX[it] = (w + vanleer64(dm, dp)) * dt;
+            } else {
+                FX[it] = tvdb_flux<R, EX>(vb[im], vb[i], vb[ip], vb[ipp], VH[it], dt);
+            }
+        }
+        return !rg.ok();
+    };
+    if constexpr (sizeof(R) == 8) {
+        if (__syncthreads_or(rows(std::true_type{})))
+            rows(std::false_type{});
+    } else {
+        rows(std::false_type{});
     }
     __syncthreads();
     // Phase 6: b - (flux - flux(i-1)) (C/tvdb.c:79-88) into VR.

@@ -60,3 +60,34 @@ def test_exact_face_velocity_near_the_largest_float(shape, mhd, cuda, oracle32):
     _, bo = oracle_ops(oracle32, u, b, bin_, shape, 1e-38)
     assert np.isfinite(bo).all() and not np.array_equal(bo, bin_)
     assert same_bits(gpu_ops(mhd, cuda, u, b, bin_, shape, 1e-38, exact=True)[1], bo)
+
+
+# momenta, energies and fields of 2^lo .. 2^hi around ordinary densities: products of two
+# differences underflow (-560), subnormals (-1070), products on the edge of the largest
+# double (505), sums beyond it (1000)
+@pytest.mark.parametrize("lo,hi", [(-560, -480), (-1070, -1000), (505, 515), (1000, 1023)])
+@pytest.mark.parametrize("shape", [(32, 8, 4), (20, 5, 3), (33, 4, 2), (64, 6, 3)])
+def test_fp64_operators_at_the_limits(shape, lo, hi, mhd, cuda, oracle64):
+    """FP64 keeps the reference's bits where the forms with fewer operations do not hold."""
+    nc, rng = cells(shape, lo, hi)
+    with np.errstate(over="ignore"):
+        u, b, bin_ = (rng.standard_normal((nc, k)) * 2.0 ** rng.uniform(lo, hi, (nc, k)) for k in (5, 3, 3))
+    u[:, 0] = 2.0 ** rng.uniform(-3, 3, nc)
+    for x in (u[:, 1:], b, bin_):
+        x[rng.random(x.shape) < 0.02] = 0
+    u, b, bin_ = u.ravel(), b.ravel(), bin_.ravel()
+    uo, bo = oracle_ops(oracle64, u, b, bin_, shape, DT)
+    gu, gb = gpu_ops(mhd, cuda, u, b, bin_, shape, DT, fp64=True)
+    assert same_bits(gu, uo) and same_bits(gb, bo)
+
+
+@pytest.mark.parametrize("dt", [0.0, 5e-324, 1e-300, 1e300])
+def test_fp64_operators_with_extreme_steps(dt, mhd, cuda, oracle64):
+    shape = (24, 5, 3)
+    nc, rng = cells(shape, dt)
+    u, b, bin_ = (rng.standard_normal((nc, k)) for k in (5, 3, 3))
+    u[:, 0] = 2.0 ** rng.uniform(-3, 3, nc)
+    u, b, bin_ = u.ravel(), b.ravel(), bin_.ravel()
+    uo, bo = oracle_ops(oracle64, u, b, bin_, shape, dt)
+    gu, gb = gpu_ops(mhd, cuda, u, b, bin_, shape, dt, fp64=True)
+    assert same_bits(gu, uo) and same_bits(gb, bo)
