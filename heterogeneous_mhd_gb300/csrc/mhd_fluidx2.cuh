@@ -443,8 +443,8 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
                     // power of two.  The flux is kept undivided (2 flux; the half goes into
                     // the step below).
                     const R pr = dmn * dm[m][s], pl = dln * dl[m][s];
-                    const R dfr = mul_if_pos(pr, pr, fast_rcp(dmn + dm[m][s]));
-                    const R d = sub_if_pos(pl, dfr, fast_div(pl, dln + dl[m][s]));
+                    const R dfr = mul_if_pos(pr, pr, rcp_ftz(dmn + dm[m][s]));
+                    const R d = sub_if_pos(pl, dfr, __fmul_rn(pl, rcp_ftz(dln + dl[m][s])));
                     flux[m][s] = (fr[m][s] - gn) + d;
                 }
             }

@@ -31,16 +31,8 @@ __device__ __forceinline__ float rabs<float>(float x)
     return fabsf(x);
 }
 
-// FAST-policy division, reciprocal and square root: the SFU approximations
-// (a few ulp) in FP32, IEEE in FP64.  The FP32 forms are the flush-to-zero
-// ones: without it each costs a range test and two scalings around the SFU
-// instruction (three of the about five instructions of a quotient).  Only
-// subnormal denominators could tell the difference, and none reaches a result:
-// densities are normal, and a limiter quotient is used only where the product
-// of its two differences is positive, so their sum is at least 2^-75.
-// The fluidx and advectbyzx kernels are bound by instruction issue: with
-// these, mul_if_pos and the kept field (mhd_fluidx2.cuh) four 256^3 steps take
-// 10.03 ms plain and 8.66 ms fused, against 10.94 and 9.27 ms before, bit for bit.
+// FAST-policy division, reciprocal and square root: CUDA's approximate forms (a few ulp)
+// in FP32, subnormal operands included (a thin or cold gas has them), IEEE in FP64.
 template <typename R>
 __device__ __forceinline__ R fast_rcp(R x)
 {
@@ -49,9 +41,7 @@ __device__ __forceinline__ R fast_rcp(R x)
 template <>
 __device__ __forceinline__ float fast_rcp<float>(float x)
 {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
+    return __fdividef(1.0f, x);
 }
 template <typename R>
 __device__ __forceinline__ R fast_div(R x, R y)
@@ -61,7 +51,7 @@ __device__ __forceinline__ R fast_div(R x, R y)
 template <>
 __device__ __forceinline__ float fast_div<float>(float x, float y)
 {
-    return __fmul_rn(x, fast_rcp(y));
+    return __fdividef(x, y);
 }
 template <typename R>
 __device__ __forceinline__ R fast_sqrt(R x)
@@ -70,6 +60,28 @@ __device__ __forceinline__ R fast_sqrt(R x)
 }
 template <>
 __device__ __forceinline__ float fast_sqrt<float>(float x)
+{
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The approximations that flush subnormal operands and results to zero, which are
+// cheaper, where neither can matter: the limiter's quotient is used only where the
+// product of its two differences is positive, so their sum is at least 2^-75 (and above
+// 2^126 both forms give 0); the EXACT forms below start from them inside range conditions.
+// With the flushing quotient in the limiter, mul_if_pos and the kept field
+// (mhd_fluidx2.cuh) four 256^3 steps take 10.12 ms plain and 8.79 ms fused, against 10.94 and
+// 9.27 ms before, bit for bit; 9.93 and 8.62 ms with flushing forms for 1 / rho and the sound speed
+// too, which lose densities below 2^-126 and sound speeds below 2^-63.
+__device__ __forceinline__ float rcp_ftz(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ double rcp_ftz(double x) { return 1.0 / x; }
+__device__ __forceinline__ float sqrt_ftz(float x)
 {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -139,7 +151,7 @@ __device__ __forceinline__ float vanleer_exact(float a, float b)
     if (__fmul_rn(a, b) > 0.f) {
         const float a2 = __fadd_rn(a, a), s = __fadd_rn(a, b);
         const float ph = __fmul_rn(a2, b), pl = __fmaf_rn(a2, b, -ph);  // 2ab = ph + pl
-        const float y = fast_rcp(s), q = __fmul_rn(ph, y);              // q within 2^-21.6 of the quotient
+        const float y = rcp_ftz(s), q = __fmul_rn(ph, y);               // q within 2^-21.6 of the quotient
         const float e = __fmul_rn(__fadd_rn(__fmaf_rn(-q, s, ph), pl), y);
         // |q + e - quotient| <= 2^-42.6 |q| (the residual's, the product's and y's errors
         // on a correction of at most 2^-21.4 |q|), 2^-45 for lo -+ err, 2^-53 for the double
@@ -183,8 +195,8 @@ static __device__ __noinline__ float add_sqrt_wide(float a, float t) { return fl
 __device__ __forceinline__ float add_sqrt_exact(float a, float t)
 {
     float s, se, r;
-    const float s0 = fast_sqrt(t);  // within 2^-22: with the correction's own error 2^-42.5 of s0
-    const float corr = __fmul_rn(__fmaf_rn(-s0, s0, t), __fmul_rn(0.5f, fast_rcp(s0)));
+    const float s0 = sqrt_ftz(t);  // within 2^-22: with the correction's own error 2^-42.5 of s0
+    const float corr = __fmul_rn(__fmaf_rn(-s0, s0, t), __fmul_rn(0.5f, rcp_ftz(s0)));
     two_sum(a, s0, s, se);
     const bool sure = ziv_round(s, __fadd_rn(se, corr), s * 0x1p-41f, r);
     if (!(sure && s0 > 0x1p-40f && s < 0x1p60f))
@@ -206,10 +218,10 @@ __device__ __forceinline__ float cfl_exact(float v, float bb, float g, float rho
         nh = -nh;
         nl = -nl;
     }
-    const float y = fast_rcp(rho), q = __fmul_rn(nh, y);
+    const float y = rcp_ftz(rho), q = __fmul_rn(nh, y);
     const float e = __fmul_rn(__fadd_rn(__fmaf_rn(-q, rho, nh), nl), y);
-    const float s0 = fast_sqrt(q);
-    const float corr = __fmul_rn(__fadd_rn(__fmaf_rn(-s0, s0, q), e), __fmul_rn(0.5f, fast_rcp(s0)));
+    const float s0 = sqrt_ftz(q);
+    const float corr = __fmul_rn(__fadd_rn(__fmaf_rn(-s0, s0, q), e), __fmul_rn(0.5f, rcp_ftz(s0)));
     two_sum(v, s0, s, se);
     // the quotient within 2^-42.6, the root within half of that and 2^-44 (corr up to 2^-21)
     const bool sure = ziv_round(s, __fadd_rn(se, corr), s * 0x1p-40f, r);
@@ -320,7 +332,7 @@ __device__ __forceinline__ R vanleer(R a, R b)
         return r;
     } else {  // branch-free: quotient for every cell, then the select
         const R ab = a * b;
-        const R q = fast_div(R(2) * ab, a + b);
+        const R q = R(2) * ab * rcp_ftz(a + b);
         return (ab > R(0)) ? q : R(0);
     }
 }
@@ -453,7 +465,7 @@ __device__ __forceinline__ R tvdb_face(R mm, R mc, R rm, R rc)
     if constexpr (EX)
         return (mm + mc) / (rm + rc);
     else
-        return r_mul(r_add(mm, mc), fast_rcp(r_add(rm, rc)));
+        return fast_div(r_add(mm, mc), r_add(rm, rc));
 }
 
 // 1-2-1 smoothing of the face velocity (C/advectbyzxA1.c:36-41): vm, v, vp at i-1, i, i+1.
@@ -533,7 +545,7 @@ __device__ __forceinline__ R tvdb_flux(R vbm, R vb0, R vbp, R vbpp, R vh, R dt)
         const R dp = r_sub(vbp, up ? vb0 : vbpp);
         const R dm = r_sub(vb0, up ? vbm : vbp);
         const R p = r_mul(dm, dp);
-        return r_mul(r_add(w, mul_if_pos(p, p, fast_rcp(r_add(dm, dp)))), dt);
+        return r_mul(r_add(w, mul_if_pos(p, p, rcp_ftz(r_add(dm, dp)))), dt);
     }
 }
 
