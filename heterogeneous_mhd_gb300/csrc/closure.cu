@@ -1436,9 +1436,8 @@ int launch_conv(const void* x, const void* w, const float* bias, void* y, void* 
     const long long ntiles = (long long)nb * (n / TX) * (n / TY) * (n / TZ);
     const int per_sm = smem > 110 * 1024 ? 1 : 2;
     const long long grid = ntiles < (long long)sms() * per_sm * 2 ? ntiles : (long long)sms() * per_sm * 2;
-    mhd::launch_after(k_conv<CIN, COUT, KS, EPI>, (unsigned)grid, 128, smem, s, static_cast<const bf16*>(x),
-        static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave), static_cast<const bf16*>(zprev), n, ntiles);
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_conv<CIN, COUT, KS, EPI>, (unsigned)grid, 128, smem, s, static_cast<const bf16*>(x),
+        static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave), static_cast<const bf16*>(zprev), n, ntiles));
 }
 
 int* g_tc_err = nullptr;  // device error word of the tcgen05 kernels
@@ -1477,10 +1476,9 @@ int launch_conv_tc2(const void* x, const void* w, const float* bias, void* y, vo
     }
     const long long ntiles = (long long)nb * (n / TCX) * (n / TCY) * (n / TCZ);
     const long long grid = ntiles < (long long)sms() ? ntiles : (long long)sms();
-    mhd::launch_after(k_conv_tc2<CIN, COUT, EPI>, (unsigned)grid, kTc2Warps * 32, smem, s,
+    return st(mhd::launch_after(k_conv_tc2<CIN, COUT, EPI>, (unsigned)grid, kTc2Warps * 32, smem, s,
         static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave),
-        static_cast<const bf16*>(zprev), n, ntiles, g_tc_err, g_gelu_tab, g_grad_tab);
-    return st(cudaGetLastError());
+        static_cast<const bf16*>(zprev), n, ntiles, g_tc_err, g_gelu_tab, g_grad_tab));
 }
 
 template <int CIN, int COUT, int EPI>
@@ -1506,10 +1504,9 @@ int launch_conv_tc(const void* x, const void* w, const float* bias, void* y, voi
         return MHD_ERR_NOMEM;
     const long long ntiles = (long long)nb * (n / TCX) * (n / TCY) * (n / TCZ);
     const long long grid = ntiles < (long long)sms() ? ntiles : (long long)sms();
-    mhd::launch_after(k_conv_tc<CIN, COUT, EPI>, (unsigned)grid, 256, smem, s, static_cast<const bf16*>(x),
+    return st(mhd::launch_after(k_conv_tc<CIN, COUT, EPI>, (unsigned)grid, 256, smem, s, static_cast<const bf16*>(x),
         static_cast<const bf16*>(w), bias, y, static_cast<bf16*>(zsave), static_cast<const bf16*>(zprev), n,
-        ntiles, g_tc_err);
-    return st(cudaGetLastError());
+        ntiles, g_tc_err));
 }
 
 bool use_tc(int n) { return !g_tc_disabled && n % TCX == 0 && n % TCY == 0 && n % TCZ == 0; }
@@ -1540,14 +1537,12 @@ int launch_wgrad(const void* a, const void* dz, float* part, float* dw, int cor,
     const long long nsets = ntiles < (long long)sms() * 2 ? ntiles : (long long)sms() * 2;
     const long long resident = (long long)sms() * (KS == 1 ? 2 : 1);  // CTAs an SM holds: by registers, by shared memory
     const long long grid = nsets < resident ? nsets : resident;
-    mhd::launch_after(k_wgrad<CIN, COUTP, KS>, (unsigned)grid, S::THREADS, smem, s, static_cast<const bf16*>(a),
-        static_cast<const bf16*>(dz), part, n, ntiles, (int)nsets);
-    if (cudaGetLastError() != cudaSuccess)
+    if (mhd::launch_after(k_wgrad<CIN, COUTP, KS>, (unsigned)grid, S::THREADS, smem, s, static_cast<const bf16*>(a),
+                          static_cast<const bf16*>(dz), part, n, ntiles, (int)nsets) != cudaSuccess)
         return MHD_ERR_CUDA;
     const size_t len = (size_t)cor * S::TAPS * cir;
-    mhd::launch_after(k_wsum, (unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s, part, (int)(nsets * S::WK),
-        S::TAPS, COUTP, CIN, cor, cir, dw);
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_wsum, (unsigned)((len + 31) / 32), kWsumWarps * 32, 0, s, part, (int)(nsets * S::WK),
+        S::TAPS, COUTP, CIN, cor, cir, dw));
 }
 
 bool shape_ok(int nb, int n) { return nb > 0 && n >= 8 && n % 8 == 0 && n <= 1024; }
@@ -1651,12 +1646,11 @@ extern "C" MHD_API int mhd_cl_colsum(const void* x, int channels, long long coun
     const int threads = 256, blocks = 256;  // blocks: the scratch holds 256 * channels partials
     if (reinterpret_cast<uintptr_t>(x) & 15)
         return MHD_ERR_ARG;  // rows are read as 16-byte chunks
-    mhd::launch_after(k_colsum, blocks, threads, 0, s, static_cast<const bf16*>(x), channels, (size_t)count, scratch);
-    if (cudaGetLastError() != cudaSuccess)
+    if (mhd::launch_after(k_colsum, blocks, threads, 0, s, static_cast<const bf16*>(x), channels, (size_t)count,
+                          scratch) != cudaSuccess)
         return MHD_ERR_CUDA;
-    mhd::launch_after(k_sum_parts, (unsigned)((nout + 31) / 32), kSumWarps * 32, 0, s, scratch, blocks,
-        (size_t)channels, (size_t)nout, out);
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_sum_parts, (unsigned)((nout + 31) / 32), kSumWarps * 32, 0, s, scratch, blocks,
+        (size_t)channels, (size_t)nout, out));
 }
 
 extern "C" MHD_API int mhd_cl_loss(const float* out, const void* target, void* dout, float* rb_scratch,
@@ -1671,16 +1665,14 @@ extern "C" MHD_API int mhd_cl_loss(const float* out, const void* target, void* d
     const size_t nv = (size_t)nb * n * n * n;
     const float gscale = 2.0f / (8.0f * (float)nv);
     const unsigned blocks = 512;
-    mhd::launch_after(k_loss1, blocks, 256, 0, s, out, static_cast<const bf16*>(target), static_cast<bf16*>(dout),
-        rb_scratch, loss_scratch, nb, n, gscale);
-    if (cudaGetLastError() != cudaSuccess)
+    if (mhd::launch_after(k_loss1, blocks, 256, 0, s, out, static_cast<const bf16*>(target), static_cast<bf16*>(dout),
+                          rb_scratch, loss_scratch, nb, n, gscale) != cudaSuccess)
         return MHD_ERR_CUDA;
-    mhd::launch_after(k_loss2, blocks_for(nv, 256), 256, 0, s, rb_scratch, static_cast<bf16*>(dout), nb, n, gscale);
-    if (cudaGetLastError() != cudaSuccess)
+    if (mhd::launch_after(k_loss2, blocks_for(nv, 256), 256, 0, s, rb_scratch, static_cast<bf16*>(dout), nb, n,
+                          gscale) != cudaSuccess)
         return MHD_ERR_CUDA;
-    mhd::launch_after(k_sum_parts, 1, kSumWarps * 32, 0, s, loss_scratch, (int)blocks, 1, 1,
-        loss);  // sum of squares; /(8N) on the host
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_sum_parts, 1, kSumWarps * 32, 0, s, loss_scratch, (int)blocks, 1, 1,
+        loss));  // sum of squares; /(8N) on the host
 }
 
 extern "C" MHD_API int mhd_cl_features(const float* u, const float* b, int n, const float* mean,
@@ -1689,9 +1681,8 @@ extern "C" MHD_API int mhd_cl_features(const float* u, const float* b, int n, co
     if (!u || !b || n <= 0 || (!raw && !x) || (x && (!mean || !inv_std)))
         return MHD_ERR_ARG;
     const size_t nv = (size_t)n * n * n;
-    mhd::launch_after(k_features, blocks_for(nv, 256), 256, 0, static_cast<cudaStream_t>(stream), u, b, n, mean,
-        inv_std, raw, static_cast<bf16*>(x));
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_features, blocks_for(nv, 256), 256, 0, static_cast<cudaStream_t>(stream), u, b, n, mean,
+        inv_std, raw, static_cast<bf16*>(x)));
 }
 
 extern "C" MHD_API int mhd_cl_normalize(const float* x, int channels, long long count, const float* mean,
@@ -1762,20 +1753,21 @@ extern "C" MHD_API int mhd_cl_apply(float* u, float* b, const float* out, int n,
         return MHD_ERR_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t nv = (size_t)n * n * n;
-    mhd::launch_after(k_apply_begin, 1, 32, 0, s, flags, esum);
+    cudaError_t e = mhd::launch_after(k_apply_begin, 1, 32, 0, s, flags, esum);
+    auto then = [&](cudaError_t r) { e = e == cudaSuccess ? r : e; };
     const unsigned blocks = blocks_for(nv, 256);
     const unsigned rblocks = blocks < 2u * (unsigned)sms() ? blocks : 2u * (unsigned)sms();  // of the reductions
-    mhd::launch_after(k_apply0, rblocks, 256, 0, s, out, nv, esum, dt, dt_min);
+    then(mhd::launch_after(k_apply0, rblocks, 256, 0, s, out, nv, esum, dt, dt_min));
     for (int a = 0; a < 3; a++) {  // the full correction, else half, else a quarter, else none
         if (a)
-            mhd::launch_after(k_apply_next, 1, 1, 0, s, flags, esum);
-        mhd::launch_after(k_apply1, rblocks, 256, 0, s, u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp,
-            esum, flags, dt, dt_min);
-        mhd::launch_after(k_apply2, blocks, 256, 0, s, u_tmp, b_tmp, n, flags, dt, dt_min);
-        mhd::launch_after(k_apply3, blocks, 256, 0, s, u, b, u_tmp, b_tmp, nv, flags, esum, ecap, fallbacks,
-            a == 2, dt, dt_min);
+            then(mhd::launch_after(k_apply_next, 1, 1, 0, s, flags, esum));
+        then(mhd::launch_after(k_apply1, rblocks, 256, 0, s, u, b, out, n, oscale, bscale, alphas[a], u_tmp, b_tmp,
+                               esum, flags, dt, dt_min));
+        then(mhd::launch_after(k_apply2, blocks, 256, 0, s, u_tmp, b_tmp, n, flags, dt, dt_min));
+        then(mhd::launch_after(k_apply3, blocks, 256, 0, s, u, b, u_tmp, b_tmp, nv, flags, esum, ecap, fallbacks,
+                               a == 2, dt, dt_min));
     }
-    return st(cudaGetLastError());
+    return st(e);
 }
 
 extern "C" MHD_API int mhd_cl_adamw(float* p, const float* g, float* m, float* v, long long count, int step, float lr,
@@ -1784,9 +1776,8 @@ extern "C" MHD_API int mhd_cl_adamw(float* p, const float* g, float* m, float* v
     if (!p || !g || !m || !v || count <= 0 || step <= 0)
         return MHD_ERR_ARG;
     const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
-    mhd::launch_after(k_adamw, blocks_for((size_t)count, 256), 256, 0, static_cast<cudaStream_t>(stream), p, g, m,
-        v, (size_t)count, lr, beta1, beta2, eps, wd, c1, c2);
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_adamw, blocks_for((size_t)count, 256), 256, 0, static_cast<cudaStream_t>(stream), p, g, m,
+        v, (size_t)count, lr, beta1, beta2, eps, wd, c1, c2));
 }
 
 extern "C" MHD_API int mhd_cl_pack(const float* w, int cout_real, int cin_real, int taps, int cout_pad, int cin_pad,
@@ -1796,7 +1787,6 @@ extern "C" MHD_API int mhd_cl_pack(const float* w, int cout_real, int cin_real, 
         (!w_fwd && !w_dgrad))
         return MHD_ERR_ARG;
     const size_t tot = (size_t)cout_pad * taps * cin_pad;
-    mhd::launch_after(k_pack, blocks_for(tot, 256), 256, 0, static_cast<cudaStream_t>(stream), w, cout_real,
-        cin_real, taps, cout_pad, cin_pad, static_cast<bf16*>(w_fwd), static_cast<bf16*>(w_dgrad));
-    return st(cudaGetLastError());
+    return st(mhd::launch_after(k_pack, blocks_for(tot, 256), 256, 0, static_cast<cudaStream_t>(stream), w, cout_real,
+        cin_real, taps, cout_pad, cin_pad, static_cast<bf16*>(w_fwd), static_cast<bf16*>(w_dgrad)));
 }

@@ -61,7 +61,7 @@ __device__ __forceinline__ void copy_strided(const V* src, V* dst, size_t n)
 
 // A launch that may start while the one before it in the stream drains; the
 // kernel begins with after_previous().  Captured into a graph it becomes a
-// programmatic edge.
+// programmatic edge.  Returns the launch's error.
 template <typename... P, typename... A>
 static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args)
 {
@@ -75,7 +75,10 @@ static cudaError_t launch_after(void (*kernel)(P...), dim3 grid, dim3 block, siz
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess)
+        (void)cudaGetLastError();  // it is the caller's: not left for whoever asks next
+    return e;
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)

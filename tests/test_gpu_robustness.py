@@ -155,3 +155,26 @@ def test_standalone_calcfl_between_steps_changes_nothing(mhd, cuda):
             assert ctx.check() == mhd.MHD_OK
         assert bitwise_equal(u, ru) and bitwise_equal(b, rb), graphs
         assert t == rt
+
+
+def test_refused_launch_leaves_no_error_behind(mhd, cuda):
+    """A launch that the runtime refuses (a transpose whose grid is beyond its limits, 70000
+    planes) is that call's error alone: the calls after it report their own."""
+    from heterogeneous_mhd_gb300 import closure
+    torch = cuda
+    cells = 70000
+    u, b = torch.zeros(5 * cells, device="cuda"), torch.zeros(3 * cells, device="cuda")
+    uo, bo = torch.empty_like(u), torch.empty_like(b)
+    w, wf = torch.zeros(32 * 27 * 32, device="cuda"), torch.empty(32 * 27 * 32, dtype=torch.bfloat16, device="cuda")
+    with mhd.Context(16, 16, 16) as ctx:
+        ctx.set_state(*mhd.init_vortex(16, 16, 16, seed=1))
+        for _ in range(2):
+            with pytest.raises(mhd.MhdError):
+                ctx.op_transpose12(uo, bo, u, b, 1, 1, cells)
+            assert ctx.divb_max() < 1e-5
+            with pytest.raises(mhd.MhdError):
+                ctx.op_transpose12(uo, bo, u, b, 1, 1, cells)
+            assert closure.cl().mhd_cl_pack(w.data_ptr(), 32, 32, 27, 32, 32, wf.data_ptr(), None,
+                                            closure.stream_ptr()) == mhd.MHD_OK
+        ctx.step(1)
+        assert ctx.check() == mhd.MHD_OK
