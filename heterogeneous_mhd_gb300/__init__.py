@@ -170,9 +170,16 @@ def _check(status: int, what: str) -> None:
         raise MhdError(status, what)
 
 
-@functools.lru_cache(maxsize=64)
 def _dims(nx, ny, nz):
     """The dimensions as the C surface takes them, by pointer (read only there)."""
+    if type(nx) is type(ny) is type(nz) is int:
+        return _int_dims(nx, ny, nz)
+    return C.byref(C.c_int(nx)), C.byref(C.c_int(ny)), C.byref(C.c_int(nz))
+
+
+@functools.lru_cache(maxsize=64)
+def _int_dims(nx, ny, nz):
+    """Plain ints only: other numbers equal to one (8.0) or held by identity (a tensor) are not it."""
     return C.byref(C.c_int(nx)), C.byref(C.c_int(ny)), C.byref(C.c_int(nz))
 
 

@@ -5,6 +5,7 @@ import re
 from pathlib import Path
 
 import numpy as np
+import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
 
@@ -88,3 +89,21 @@ def test_no_cpu_fallback_in_product():
     for p in list(pkg.rglob("*.py")) + list(pkg.rglob("*.cu")) + list(pkg.rglob("*.cuh")) + list(pkg.rglob("*.c")):
         text = p.read_text()
         assert "liboracle" not in text and "orc_" not in text and "oracle/" not in text, p
+
+
+def test_dimensions_are_taken_as_given_each_time():
+    """The drop-in operators' dimensions: what was refused before a call with an equal int is
+    refused after it, and an array is read on each call."""
+    import heterogeneous_mhd_gb300 as m
+
+    def values(*dims):
+        return [ref._obj.value for ref in m._dims(*dims)]
+
+    assert values(8, 4, 2) == [8, 4, 2] == values(np.int64(8), np.int32(4), 2)
+    for bad in (8.0, np.float32(8), "8", None):
+        with pytest.raises(TypeError):
+            m._dims(bad, 4, 2)
+    n = np.array(8)  # a 0-d integer array
+    assert values(n, 4, 2) == [8, 4, 2]
+    n[...] = 16
+    assert values(n, 4, 2) == [16, 4, 2]
