@@ -414,10 +414,18 @@ static int op_copy(mhd_ctx* c, const void* src, void* dst, size_t bytes)
     return MHD_OK;
 }
 
-// copy_matrix of u and b
+static bool overlap(const void* a, size_t na, const void* b, size_t nb)
+{
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+}
+
+// copy_matrix of u and b, u first: in one launch unless one of them is nothing to do, or the
+// second reads or writes what the first writes, or writes what it reads
 static int op_copy2(mhd_ctx* c, const void* su, void* du, size_t bu, const void* sb, void* db, size_t bb)
 {
-    if (su == du || sb == db) {
+    if (su == du || sb == db || bu == 0 || bb == 0 || overlap(du, bu, sb, bb) || overlap(du, bu, db, bb) ||
+        overlap(su, bu, db, bb)) {
         MHD_TRY(op_copy(c, su, du, bu));
         return op_copy(c, sb, db, bb);
     }

@@ -304,3 +304,42 @@ def test_fp64_ops_wide_magnitudes_vs_oracle(shape, lo, hi, mhd, cuda, oracle64):
     assert bitwise_equal(out["fluidx_u"], uo)
     assert bitwise_equal(out["advect_b"], bo)
     assert out["calcfl"][0] == oracle64.calcfl(u, b, nx, ny, nz)
+
+
+@pytest.mark.parametrize("cells", [257, 4096, 300000])
+def test_copy_of_arrays_that_overlap_is_u_then_b(cells, mhd, cuda):
+    """copy_matrix copies u, then b: b may be read from what u was copied into, written to what
+    u was read from, or written over u's copy."""
+    torch = cuda
+    n = cells
+    with mhd.Context(1, 1, 1) as ctx:
+        for _ in range(3):
+            base = torch.arange(16 * n, dtype=torch.float32, device="cuda")
+            u, uu, b, ub = base[:5 * n], base[8 * n:13 * n], base[9 * n:12 * n], base[13 * n:]
+            torch.cuda.synchronize()
+            ctx.op_copy(u, b, uu, ub, n, 1, 1)  # b lies in uu
+            ctx.sync()
+            assert torch.equal(ub, u[n:4 * n]) and torch.equal(uu, u)
+            base = torch.arange(16 * n, dtype=torch.float32, device="cuda")
+            u, uu, b, ub = base[:5 * n], base[8 * n:13 * n], base[13 * n:], base[n:4 * n]
+            want_u, want_b = u.clone(), b.clone()
+            torch.cuda.synchronize()
+            ctx.op_copy(u, b, uu, ub, n, 1, 1)  # ub lies in u
+            ctx.sync()
+            assert torch.equal(uu, want_u) and torch.equal(ub, want_b)
+            ub = base[9 * n:12 * n]
+            u.copy_(want_u)
+            torch.cuda.synchronize()
+            ctx.op_copy(u, b, uu, ub, n, 1, 1)  # ub lies in uu
+            ctx.sync()
+            want = want_u.clone()
+            want[n:4 * n] = want_b
+            assert torch.equal(uu, want)
+
+
+def test_copy_of_nothing_launches_nothing(mhd, cuda):
+    u, b = cuda.zeros(8, device="cuda"), cuda.zeros(8, device="cuda")
+    with mhd.Context(1, 1, 1) as ctx:
+        before = ctx.launch_count()
+        ctx.op_copy(u[:4], b[:4], u[4:], b[4:], 0, 1, 1)
+        assert ctx.launch_count() == before
