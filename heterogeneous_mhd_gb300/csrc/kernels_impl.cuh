@@ -138,22 +138,50 @@ static bool fluidx_range_ok(const FluidxArgs& a)
     return a.axis == 1 || plan_fluidx(a.nx, a.ny, a.use_tma != 0).C != 0;
 }
 
-// Every other pencil length, and unaligned arrays: FP32 the ragged engine
-// (mhd_ragged.cuh), FP64 one thread per cell (bound by the FP64 pipe).
-template <typename RR>
+// Where FP32 takes one thread per cell (k_fluidx, k_advect) instead of the ragged engine: short
+// pencils, which fill few of the engine's lanes, and small boxes, whose time is the latency of one
+// CTA's chain.  In both the CTAs must be filled (P pencils of n cells), or few.  Measured per launch
+// (us, engine / one thread per cell; n x m x m cells, m = 32, 64, 128):
+//   fluidx      8: 6.8/4.1 7.3/4.2 15.7/5.4;  17: 7.9/5.2 8.6/6.1 18.2/13.8;  18: 6.5/5.1 7.3/6.2 12.1/13.8;
+//              20: 6.7/3.9 7.5/4.5 16.7/10.4;  31: 8.7/5.4 10.1/8.2 20.1/21.6;  40: 6.6/4.0 7.3/7.0 15/19
+//   advectbyzx  8: 9.3/6.2 9.8/6.2 17/9.4;  12: 6.6/6.1 7.2/6.7 12/11.9;  13: 9.6/5.1 11/6.1 19/12.6;
+//              24: 6.7/6.1 8.2/8.6 13/18.6;  31: 9.8/6.4 11.7/9.0 19/23;  40: 8.1/6.8 10.3/10.3 18/29
+// 131 pencils in a row (a prime: one to a CTA) of 12 cells, 127 planes: 13/21 and 12/27.
+static bool cta_fills(int nx, int ny, int nz)
+{
+    const int P = fluidx_pencils(nx, ny);  // advect_pencils is the same
+    return P * nx >= 64 || (long long)(ny / P) * nz <= 2048;
+}
+
+constexpr long long kThreadPerCell = 200000;  // cells of a launch
+
+static bool thread_per_cell_fluidx(int nx, int ny, int nz, int boxes)
+{
+    const bool any = nx <= 17 || (nx <= 20 && nx % 3 != 0);  // of 18 cells: 24 of 24 lane slots in use
+    return (any || (nx <= 40 && (long long)nx * ny * nz * boxes <= kThreadPerCell)) && cta_fills(nx, ny, nz);
+}
+
+// Pencils of whole 16-byte pieces (multiples of 4) are staged faster by the engine.
+static bool thread_per_cell_advect(int nx, int ny, int nz, int boxes)
+{
+    const bool any = nx <= 8 || (nx <= 14 && nx % 4 != 0);
+    const long long most = (nx % 4 != 0) ? kThreadPerCell : 65536;
+    return (any || (nx <= 40 && (long long)nx * ny * nz * boxes <= most)) && cta_fills(nx, ny, nz);
+}
+
+// Every other pencil length, and unaligned arrays: the ragged engine (mhd_ragged.cuh), or one
+// thread per cell (FP64, which is bound by its pipe, and the short pencils of FP32).
 static cudaError_t fluidx_any(const FluidxArgs& a, cudaStream_t s)
 {
-    if constexpr (sizeof(RR) == 4) {
+    if (kV2 && !thread_per_cell_fluidx(a.nx, a.ny, a.nz, a.bs.count))
         return fluidx_ragged(a, EX, s);
-    } else {
-        static bool attr = false;
-        cudaError_t e = allow_smem(k_fluidx<RR, EX>, attr);
-        if (e != cudaSuccess)
-            return e;
-        dim3 grid(a.ny / a.P, a.nz, a.bs.count);
-        return launch_after(k_fluidx<RR, EX>, grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx,
-            a.P) * sizeof(RR), s, a);
-    }
+    static bool attr = false;
+    cudaError_t e = allow_smem(k_fluidx<R, EX>, attr);
+    if (e != cudaSuccess)
+        return e;
+    dim3 grid(a.ny / a.P, a.nz, a.bs.count);
+    return launch_after(k_fluidx<R, EX>, grid, fluidx_threads(a.nx, a.P), fluidx_smem_elems(a.nx, a.P) * sizeof(R), s,
+                        a);
 }
 
 static cudaError_t fluidx(const FluidxArgs& in, cudaStream_t s)
@@ -198,13 +226,13 @@ static cudaError_t fluidx(const FluidxArgs& in, cudaStream_t s)
             }
         }
     }
-    return fluidx_any<R>(a, s);
+    return fluidx_any(a, s);
 }
 
-static int fluidx_parts(int nx, int ny, int nz, int aligned)
+static int fluidx_parts(int nx, int ny, int nz, int aligned, int boxes)
 {
     const FxPlan p = plan_fluidx(nx, ny, aligned != 0);
-    if (kV2 && p.C == 0)
+    if (kV2 && p.C == 0 && !thread_per_cell_fluidx(nx, ny, nz, boxes))
         return rag_fluidx_parts(nx, ny, nz);
     return (ny / p.P) * nz;
 }
@@ -684,7 +712,7 @@ static cudaError_t advect(const AdvectArgs& in, cudaStream_t s)
             case 64: return launch_ad2<6, 64>(a, s);
             }
         }
-        if (rag_shape(a.nx, 2).C)
+        if (rag_shape(a.nx, 2).C && !thread_per_cell_advect(a.nx, a.ny, a.nz, a.bs.count))
             return advect_ragged(a, EX, s);
     }
     static bool attr = false;

@@ -158,7 +158,7 @@ static int tma_ok(const mhd_ctx* c, int nx)
 // CFL partials written by the epilogue of the step's last fluidx.
 static size_t fluidx_parts(const mhd_ctx* c)
 {
-    return (size_t)c->ks->fluidx_parts(c->nx, c->ny, c->nz, tma_ok(c, c->nx));
+    return (size_t)c->ks->fluidx_parts(c->nx, c->ny, c->nz, tma_ok(c, c->nx), 1);
 }
 
 static cudaEvent_t ev_get(mhd_ctx* c)

@@ -133,10 +133,15 @@ static void assign_worklist(mhd_batch* b)
         b->cls[ok[k]].multi = true;
 }
 
-// CFL partials per box that the step's last fluidx writes for a class
+// CFL partials per box that the step's last fluidx writes for a class, in its own launch
+static int fluidx_parts_own(const mhd_batch* b, const SizeClass& c)
+{
+    return b->ks->fluidx_parts(c.n, c.n, c.n, tma_ok(b, c.n), (int)c.boxes.size());
+}
+
 static int fluidx_parts_of(const mhd_batch* b, const SizeClass& c)
 {
-    return c.multi ? b->ks->multi_fluidx_parts(c.n) : b->ks->fluidx_parts(c.n, c.n, c.n, tma_ok(b, c.n));
+    return c.multi ? b->ks->multi_fluidx_parts(c.n) : fluidx_parts_own(b, c);
 }
 
 static BoxStrides strides(const mhd_batch* b, const SizeClass& c)
@@ -225,7 +230,7 @@ extern "C" MHD_API int mhd_batch_create(mhd_batch** out, int nboxes, const int* 
         c.side = b->elem == 4 && b->ks->batch_side_ok(c.n, (int)m);
         if (st == MHD_OK && (c.side || (b->elem == 4 && b->ks->multi_ok(c.n) && tma_ok(b, c.n))))
             st = cu(cudaMalloc(&c.W, m * c.cells() * 8));
-        const size_t pa = (c.cells() + 255) / 256 + 1, pf = (size_t)b->ks->fluidx_parts(c.n, c.n, c.n, tma_ok(b, c.n));
+        const size_t pa = (c.cells() + 255) / 256 + 1, pf = (size_t)fluidx_parts_own(b, c);
         c.part_per_box = std::max(pa, pf);
         if (b->ks->multi_ok(c.n))
             c.part_per_box = std::max(c.part_per_box, (size_t)b->ks->multi_fluidx_parts(c.n));
@@ -423,7 +428,7 @@ static int enqueue_step(mhd_batch* b, double cfl)
         BTRY(T(1, U1, B1, U0, B0, W1));
         BTRY(A(B0, B1, U1, B1, W1));
         BTRY(F(U0, U1, B0, c.part, nullptr));  // with the CFL partials of the next step
-        c.cfl_nparts = b->ks->fluidx_parts(n, n, n, tma_ok(b, n));
+        c.cfl_nparts = fluidx_parts_own(b, c);
     }
     return enqueue_multi(b, cfl);
 }

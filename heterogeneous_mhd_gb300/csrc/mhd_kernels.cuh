@@ -176,12 +176,17 @@ __device__ __forceinline__ R warp_max(R x)
 // NaN (find_max, C/mhdflux.c:61-72); the values are non-negative, so their bits
 // are ordered as they are.  Contains one __syncthreads; red must not be read by a
 // previous call that is not separated by another barrier.
-__device__ __forceinline__ double pencil_max64(double x, double* red, int n, int lp)
+template <typename R>
+__device__ __forceinline__ R pencil_max(R x, R* red, int n, int lp)
 {
-    using U = unsigned long long;
+    using U = std::conditional_t<sizeof(R) == 8, unsigned long long, unsigned>;
     auto top = [](U a, U b) { return a > b ? a : b; };
-    U m = (U)__double_as_longlong(x) & 0x7fffffffffffffffULL;
-    m = m > 0x7ff0000000000000ULL ? 0 : m;  // NaN
+    U m;
+    if constexpr (sizeof(R) == 8)
+        m = (U)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+    else
+        m = (U)__float_as_int(x) & 0x7fffffffU;
+    m = m > (sizeof(R) == 8 ? (U)0x7ff0000000000000ULL : (U)0x7f800000U) ? 0 : m;  // NaN
     U* r = reinterpret_cast<U*>(red);
     U c = 0;
     if ((n & 31) == 0) {
@@ -201,7 +206,10 @@ __device__ __forceinline__ double pencil_max64(double x, double* red, int n, int
         for (int s = 0; s < n; s++)
             c = top(c, row[s]);
     }
-    return __longlong_as_double((long long)c);
+    if constexpr (sizeof(R) == 8)
+        return __longlong_as_double((long long)c);
+    else
+        return __int_as_float((int)c);
 }
 
 // --------------------------------------------------------------- staging
@@ -242,8 +250,8 @@ __host__ __device__ inline size_t fluidx_smem_elems(int n, int P)
 // neighbour stencil is exchanged through shared memory between barriers.
 // Optionally (cfl_part != nullptr) the epilogue evaluates calcfl's per-cell
 // speed on the new u and the face b, and writes one partial max per CTA.
-// FP64 only (the FP32 lengths without a fixed engine: mhd_ragged.cuh), bound by
-// the FP64 pipe: one thread per cell and plain exchanges cost nothing beside it.
+// FP64 (bound by the FP64 pipe: one thread per cell and plain exchanges cost nothing
+// beside it) and the short pencils of FP32 (thread_per_cell, kernels_impl.cuh).
 template <typename R, bool EX>
 __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
 {
@@ -333,10 +341,12 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
             if constexpr (FEW) {
                 rg.see(w[4]);
                 cell_flux64(w, f, v, ci);
+            } else if constexpr (sizeof(R) == 4 && !EX) {
+                cell_flux_pinned(w, f, v, ci);
             } else {
                 cell_flux<R, EX>(w, f, v, ci);
             }
-            const R c = pencil_max64(ci, red, n, lp);
+            const R c = pencil_max<R>(ci, red, n, lp);
             scale_flux<R, EX>(v, c);
 #pragma unroll
             for (int s = 0; s < 5; s++) {
@@ -427,12 +437,20 @@ __global__ void __launch_bounds__(512) k_fluidx(FluidxArgs a)
             q[s] = advance(q[s], -dt, flux[s], xa[5 * mem + s]);
         return !rg.ok();
     };
-    if (__syncthreads_or(sweep(std::true_type{})))
+    if constexpr (sizeof(R) == 8) {
+        if (__syncthreads_or(sweep(std::true_type{})))
+            sweep(std::false_type{});
+    } else {
         sweep(std::false_type{});
+    }
 #pragma unroll
     for (int s = 0; s < 5; s++)
         if (act)
             su[5 * me + s] = q[s];  // own slot: no other thread reads su after staging
+    if constexpr (sizeof(R) == 4)
+        if (act && a.w_out)
+            reinterpret_cast<float2*>(a.w_out)[c0 + me] = make_float2(q[0], q[1]);
+    before_next();
 
     // ---- optional calcfl epilogue on the new state
     if (a.cfl_part) {

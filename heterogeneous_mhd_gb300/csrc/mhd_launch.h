@@ -24,7 +24,7 @@ struct KernelSet {
     cudaError_t (*divb)(const void* b, int nx, int ny, int nz, double* part, int* nparts, cudaStream_t);
     size_t part_bytes; // sizeof(CflPart<R>)
     // number of CTAs (= CFL partials of the epilogue) of a fluidx launch
-    int (*fluidx_parts)(int nx, int ny, int nz, int aligned);
+    int (*fluidx_parts)(int nx, int ny, int nz, int aligned, int boxes);
     // nonzero if the sweeps along y and z of the fused step have kernels for this grid
     int (*fused_ok)(int nx, int ny, int nz);
     // nonzero if the x-sweep fluidx of this grid writes the (rho, m_x) side array (FluidxArgs::w_out)

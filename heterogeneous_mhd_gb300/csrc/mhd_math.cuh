@@ -276,8 +276,9 @@ __device__ __forceinline__ double vanleer64(double a, double b)
     return r;
 }
 
-// cell_flux (below) in FP64
-__device__ __forceinline__ void cell_flux64(const double q[5], const double f[3], double v[5], double& ci)
+// cell_flux (below) in FP64 (R = double)
+template <typename R>
+__device__ __forceinline__ void cell_flux64(const R q[5], const R f[3], R v[5], R& ci)
 {
     constexpr double gamma = 5.0 / 3.0, k2 = (2.0 - gamma) / 2.0;
     static_assert(k2 * 2.0 == 2.0 - gamma, "the half is exact");
@@ -382,6 +383,30 @@ __device__ __forceinline__ void cell_flux(const R q[5], const R f[3], R v[5], R&
         const R p = ps - R(0.5) * bb;
         ci = rabs(vx) + fast_sqrt(rabs((bb + gamma * p) * ri));
     }
+}
+
+// cell_flux in FAST for the two kernels that share pencil lengths (k_fluidx and k_fluidx_rag, by
+// the size of the box): which products go into a multiply-add is written out where it was found to
+// depend on the code around the call, so both give the same bits.  (Found by comparing the
+// outputs of the 64 ways to write them with those of the kernel that took these lengths first;
+// a run that feeds the state to the closure net needs it: the net amplifies a last-bit change by 1e5.)
+__device__ __forceinline__ void cell_flux_pinned(const float q[5], const float f[3], float v[5], float& ci)
+{
+    constexpr float kG1 = kGammaF - 1.0f, kK = 0.5f * (2.0f - kGammaF);
+    const float ri = fast_rcp(q[0]);
+    const float vx = q[1] * ri;
+    const float mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
+    const float p0 = __fmul_rn(f[0], f[0]);
+    const float bb = __fmaf_rn(f[2], f[2], __fmaf_rn(f[1], f[1], p0));
+    const float ps = __fmaf_rn(kK, bb, __fmul_rn(q[4] - 0.5f * mm * ri, kG1));
+    v[0] = q[1];
+    v[1] = __fsub_rn(__fmaf_rn(q[1], vx, ps), p0);
+    v[2] = q[2] * vx - f[1] * f[0];
+    v[3] = q[3] * vx - f[2] * f[0];
+    const float dot = __fmaf_rn(f[2], q[3], __fmaf_rn(f[0], q[1], __fmul_rn(f[1], q[2])));
+    v[4] = __fmaf_rn(__fadd_rn(q[4], ps), vx, -__fmul_rn(__fmul_rn(f[0], dot), ri));
+    const float p = ps - 0.5f * bb;
+    ci = fabsf(vx) + fast_sqrt(fabsf((bb + kGammaF * p) * ri));
 }
 
 // Divide the flux by the pencil max when it is positive (C/mhdflux.c:48-57).

@@ -221,29 +221,6 @@ __device__ __forceinline__ void rag_lds(const float* s, float (&d)[NF])
     }
 }
 
-// cell_flux's FAST form with the roundings that k_fluidx, the kernel of these lengths
-// before, was compiled to (which products went into a multiply-add): the two agree bit for
-// bit, which a run that feeds the state to the closure net needs (the net amplifies a
-// last-bit change by 1e5).
-__device__ __forceinline__ void rag_cell_flux(const float q[5], const float f[3], float v[5], float& ci)
-{
-    constexpr float kG1 = kGammaF - 1.0f, kK = 0.5f * (2.0f - kGammaF);
-    const float ri = fast_rcp(q[0]);
-    const float vx = q[1] * ri;
-    const float mm = q[1] * q[1] + q[2] * q[2] + q[3] * q[3];
-    const float p0 = __fmul_rn(f[0], f[0]);
-    const float bb = __fmaf_rn(f[2], f[2], __fmaf_rn(f[1], f[1], p0));
-    const float ps = __fmaf_rn(kK, bb, __fmul_rn(q[4] - 0.5f * mm * ri, kG1));
-    v[0] = q[1];
-    v[1] = __fsub_rn(__fmaf_rn(q[1], vx, ps), p0);
-    v[2] = q[2] * vx - f[1] * f[0];
-    v[3] = q[3] * vx - f[2] * f[0];
-    const float dot = __fmaf_rn(f[2], q[3], __fmaf_rn(f[0], q[1], __fmul_rn(f[1], q[2])));
-    v[4] = __fmaf_rn(__fadd_rn(q[4], ps), vx, -__fmul_rn(__fmul_rn(f[0], dot), ri));
-    const float p = ps - 0.5f * bb;
-    ci = fabsf(vx) + fast_sqrt(fabsf((bb + kGammaF * p) * ri));
-}
-
 // CTAs per SM that k_fluidx_rag is bounded to in FAST (0: as the compiler finds): the kinds whose
 // registers pass the next CTA's share (128 instead of 96, 79 instead of 72) without a bound and
 // hold in it without spills (pencils of 72 cells, four CTAs instead of five: 14.6 against 10.6 us).
@@ -341,7 +318,7 @@ __global__ void __launch_bounds__(kRagThreads, EX ? 0 : rag_fluidx_ctas(C, D)) k
             if constexpr (EX)
                 cell_flux<R, EX>(w[m], f[m], v[m], ci);
             else
-                rag_cell_flux(w[m], f[m], v[m], ci);
+                cell_flux_pinned(w[m], f[m], v[m], ci);
             cm = fmaxf(cm, ci);
         }
         const R c = g.max(cm, rd);

@@ -96,3 +96,48 @@ def test_ragged_steps_vs_oracle(shape, mhd, cuda, oracle32):
         ctx.step(3, cfl=0.7)
         gu, gb = ctx.get_state()
         assert rel_l2(gu, ref[0]) < 1e-5 and rel_l2(gb, ref[1]) < 1e-5
+
+
+# Short pencils and small boxes take one thread per cell, unless the CTAs would hold one short
+# pencil each (127 rows, a prime) and be many: the engine's groups of 8 and 16 lanes there.
+@pytest.mark.parametrize("n", [n for n in range(3, 41) if n not in (4, 8, 10, 22, 25, 28, 31, 35, 38)])
+def test_ragged_short_pencils_in_a_large_box_vs_oracle(n, mhd, cuda, oracle32):
+    torch = cuda
+    ny, nz = 127, 17
+    u, b, bin_ = state(n, ny, nz, 3 * n, mhd)
+    uo, bo = np.full_like(u, 7), bin_.copy()
+    oracle32.fluidx(uo, b.copy(), n, ny, nz, DT, u.copy(), b.copy())
+    oracle32.advectbyzx(u.copy(), bo, n, ny, nz, DT, u.copy(), b.copy())
+    for exact in (True, False):
+        for off in (0, 1):
+            with mhd.Context(1, 1, 1, exact=exact) as ctx:
+                du, db = shifted(torch, u, off), shifted(torch, b, off)
+                ou, ob = shifted(torch, np.full_like(u, 7), off), shifted(torch, bin_, off)
+                ctx.op_fluidx(ou, du, db, n, ny, nz, DT)
+                ctx.op_advectbyzx(ob, du, db, n, ny, nz, DT)
+                ctx.sync()
+                gu, gb = ou.cpu().numpy(), ob.cpu().numpy()
+            if exact:
+                assert bitwise_equal(gu, uo) and bitwise_equal(gb, bo), off
+            else:
+                assert rel_l2(gu, uo) < FAST_OP_TOL and rel_l2(gb, bo) < FAST_OP_TOL, off
+
+
+@pytest.mark.parametrize("edge,boxes", [(15, 64), (18, 40), (20, 10), (21, 24), (30, 8), (33, 6), (40, 4)])
+@pytest.mark.parametrize("exact", [False, True])
+def test_engine_and_thread_per_cell_give_the_same_steps(edge, boxes, exact, mhd, cuda):
+    """A box steps bit for bit alike alone (one thread per cell) and among so many that the
+    engine takes them, in both policies."""
+    ics = [mhd.init_vortex(edge, edge, edge, seed=s) for s in range(boxes)]
+    with mhd.Batch([edge] * boxes, exact=exact) as bt:
+        for i, (u, b) in enumerate(ics):
+            bt.set_box(i, u, b)
+        bt.step(3)
+        bt.sync()
+        got = [bt.get_box(i) for i in range(boxes)]
+    for i in (0, boxes - 1):
+        with mhd.Context(edge, edge, edge, exact=exact) as ctx:
+            ctx.set_state(*ics[i])
+            ctx.step(3)
+            u, b = ctx.get_state()
+        assert bitwise_equal(got[i][0], u) and bitwise_equal(got[i][1], b)
