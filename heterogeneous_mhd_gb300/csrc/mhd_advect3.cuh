@@ -228,12 +228,6 @@ __global__ void __launch_bounds__(384) k_advect3(AdvectArgs a)
                 bv[m] = (r <= J) ? bb[3 * m + BJ] : bb[3 * m + BK];
                 b1own[m] = bb[3 * m + BD];
             }
-            if (AX == 0 && b1s != ub && live && r < J) {  // early: its latency passes behind the row's work
-                ldg_chunk<float, C * 3>(b1s + (((size_t)(k % nz) * ny + j0 + r) * n + g.t * C) * 3, bb);
-#pragma unroll
-                for (int m = 0; m < C; m++)
-                    b1own[m] = bb[3 * m];
-            }
             tvdb_row<R, EX, C, T>(g, vr, bv, dt, seam, F, bn);
         }
         const int pk = k & 1, pk1 = (k + 1) & 1;
@@ -249,6 +243,13 @@ __global__ void __launch_bounds__(384) k_advect3(AdvectArgs a)
         // ---- combine and store the owned pencils (A-row groups 0..J-1)
         if (live && r < J) {
             const size_t cell0 = ((size_t)(k % nz) * ny + j0 + r) * n + g.t * C;
+            if (AX == 0 && b1s != ub) {  // (read before the row's work, its registers cost a CTA per SM)
+                float b1c[C * 3];
+                ldg_chunk<float, C * 3>(b1s + cell0 * 3, b1c);
+#pragma unroll
+                for (int m = 0; m < C; m++)
+                    b1own[m] = b1c[3 * m];
+            }
             float fa1[C], fb[C], fbp[C], b3[C];  // 16-byte loads: no bank conflicts for C = 4
             lds_chunk<float, C>(FA + (size_t)(r + 1) * n + g.t * C, fa1);
             lds_chunk<float, C>(FB + ((size_t)pk * J + r) * n + g.t * C, fb);
