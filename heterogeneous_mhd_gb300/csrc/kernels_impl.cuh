@@ -454,22 +454,22 @@ struct A6Plan {
     int C, J, K, T;
 };
 
-// Planes per CTA: the divisor K of nz up to 64 with the least waves x (K + 1.5), a
-// wave being the CTAs that fit at once (by registers: 10, 8, 6, 5, 5 per SM for C = 2,
-// 3, 4, 6, 8) and 1.5 planes what a CTA spends on two plane loads and a B row before
-// its first plane.  Measured per launch (K = 1, 2, 4, 8, 16, 32): 64^3 11, 9.7, 10.7, 14;
-// 96^3 18.5, 16.9, 15.1, 17; 128^3 36, 29, 25.9, 26.1; 192^3 103, 79, 66, 60, 64;
-// 256^3 -, -, -, 119, 116, 123 us: the rule takes the best of each.
-static int a6_planes(int C, int ny, int nz, int J, int boxes)
+// Planes per CTA: the divisor K of the launch's planes nk up to 64 with the least waves x
+// (K + 1.5), a wave being the CTAs that fit at once (by registers: 10, 8, 6, 5, 5 per SM for
+// C = 2, 3, 4, 6, 8) and 1.5 planes what a CTA spends on two plane loads and a B row before
+// its first plane.  Measured per launch (us, K = 1, 2, 4, 8, 16, 32): 32^3 8.1, 8.5, 10.3, 13;
+// 64^3 11.3, 10.0, 10.2, 14; 96^3 18.6, 16.5, 14.9, 16.8, 22; 128^3 36, 29, 26.0, 26.2, 24.8,
+// 39; 192^3 103, 80, 67, 61.3, 64.9, 65.6; 256^3 203, 154, 132, 119.5, 117.0, 124.  The rule takes
+// 1, 2, 4, 4, 32 and 16: the best or within 5% of it, 7% at 192^3.
+static int a6_planes(int per_sm, int ny, int nk, int J, int boxes)
 {
-    const int per_sm = (J > 2) ? 3 : (C == 2 ? 10 : (C == 3 ? 8 : (C == 4 ? 6 : 5)));
     const long long wave = 152LL * per_sm;
     int K = 1;
     long long best = -1;
-    for (int k = 1; k <= nz && k <= 64; k++) {
-        if (nz % k != 0)
+    for (int k = 1; k <= nk && k <= 64; k++) {
+        if (nk % k != 0)
             continue;
-        const long long ctas = (long long)(ny / J) * (nz / k) * boxes;
+        const long long ctas = (long long)(ny / J) * (nk / k) * boxes;
         const long long cost = (ctas + wave - 1) / wave * (2 * k + 3);
         if (best < 0 || cost < best) {
             best = cost;
@@ -497,7 +497,9 @@ static bool plan_advect6(const AdvectArgs& a, bool aligned, A6Plan& p)
     if (a.ny % p.J != 0)
         return false;
     const int kt = tune_value(TUNE_ADVECT_K);
-    p.K = (kt > 0 && kt <= 64) ? (a.nz % kt == 0 ? kt : 0) : a6_planes(p.C, a.ny, a.nz, p.J, a.bs.count);
+    const int nk = a.kcount ? a.kcount : a.nz;  // a slab's launches are planned for the slab
+    const int per_sm = (p.J > 2) ? 3 : (p.C == 2 ? 10 : (p.C == 3 ? 8 : (p.C == 4 ? 6 : 5)));
+    p.K = (kt > 0 && kt <= 64) ? (nk % kt == 0 ? kt : 0) : a6_planes(per_sm, a.ny, nk, p.J, a.bs.count);
     return p.K != 0;
 }
 
@@ -840,9 +842,10 @@ static int tail_slabs_ok(int nx, int ny, int nz, int kcount)
     a.nx = nx;
     a.ny = ny;
     a.nz = nz;
+    a.kcount = kcount;
     a.ub = a.b1_src = a.w = reinterpret_cast<const void*>(uintptr_t(256));
     A6Plan p6;
-    return (plan_advect6(a, aligned, p6) && kcount % p6.K == 0) ? 1 : 0;
+    return plan_advect6(a, aligned, p6) ? 1 : 0;
 }
 
 static int batch_side_ok(int n, int boxes)

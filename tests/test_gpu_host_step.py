@@ -121,3 +121,17 @@ def test_step_host_fused_tail_in_slabs(shape, exact, mhd, cuda):
         assert same_clock(ctx.time(), tr)
     # 8 chunked CFL passes, a whole step (13 launches), a step whose tail is 3 x 8 slab launches
     assert launches >= 8 + 13 + 10 + 24, launches
+
+
+@pytest.mark.parametrize("shape", [(32, 64, 64), (96, 64, 128), (192, 64, 64), (256, 32, 64), (128, 128, 32)])
+@pytest.mark.parametrize("exact", [False, True])
+def test_step_host_slab_launches_of_every_length(shape, exact, mhd, cuda):
+    """The fused tail in slabs, whose advectbyzx is planned for the slab's planes."""
+    u0, b0 = mhd.init_vortex(*shape, seed=11)
+    ur, br, tr, _ = three_calls(mhd, u0, b0, shape, 2, True, exact)
+    with mhd.Context(*shape, exact=exact) as ctx:
+        u, b = u0.copy(), b0.copy()
+        ctx.step_host(u, b, 2, cfl=0.7, fused=True)
+        assert ctx.check() == mhd.MHD_OK
+        assert bitwise_equal(u, ur) and bitwise_equal(b, br)
+        assert same_clock(ctx.time(), tr)
