@@ -883,13 +883,18 @@ static int multi_fluidx_parts(int n)
 // largest K <= 64 that leaves the class kMultiAdCtas CTAs.  The classes of a launch fill
 // its waves together, so a class needs no waves of its own and a larger K saves the
 // CTAs' prologues (24 boxes, five steps: 12.67 ms with 3040 CTAs per class, 11.56
-// with 1000, 11.35 with 500, 11.36 with 250).
+// with 1000, 11.35 with 500, 11.36 with 250).  A class alone in its launch has
+// only its own waves (six CTAs an SM): the largest K within 10% of the least waves x (K + 1.5)
+// (a6_planes): 46 boxes of 48^3, three steps, 3.64 ms, 3.90 with the 500; 4 of 64^3 0.73 with both.
 constexpr long long kMultiAdCtas = 500;
-static int multi_advect_k(int n, int count)
+static int multi_advect_k(int n, int count, int nseg)
 {
+    auto ctas = [&](int k) { return (long long)(n / kMultiAdJ) * (n / k) * count; };
+    auto cost = [&](int k) { return (ctas(k) + 911) / 912 * (2 * k + 3); };
+    const long long most = cost(a6_planes(6, n, n, kMultiAdJ, count)) * 11 / 10;
     int K = 1;
     for (int k = 1; k <= n && k <= 64; k++)
-        if (n % k == 0 && (long long)(n / kMultiAdJ) * (n / k) * count >= kMultiAdCtas)
+        if (n % k == 0 && (nseg == 1 ? cost(k) <= most : ctas(k) >= kMultiAdCtas))
             K = k;
     return K;
 }
@@ -964,7 +969,7 @@ static cudaError_t advect_multi(const AdvectArgs* in, int nseg, cudaStream_t s)
             if (!a.w || (al & 15) != 0 || a.b1_src != a.ub || a.axis != 0 || a.kcount != 0 || a.kbeg != 0 ||
                 (a.bs.count != 1 && a.bs.w != cells * 8))
                 return cudaErrorInvalidValue;
-            const int K = multi_advect_k(n, a.bs.count);
+            const int K = multi_advect_k(n, a.bs.count, nseg);
             m.a[i] = a;
             m.a[i].P = kMultiAdJ;
             m.a[i].K = K;
