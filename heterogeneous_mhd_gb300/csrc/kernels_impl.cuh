@@ -805,20 +805,37 @@ static int fused_ok(int nx, int ny, int nz)
     return plan_fluidx_sweep(ny, nx, 1, p) && plan_fluidx_sweep(nz, nx, 1, p) && advect_ok(1) && advect_ok(2);
 }
 
-// nonzero if the x-sweep fluidx of this grid writes the (rho, m_x) side array
-// when asked: every FP32 kernel does
-static int fluidx_writes_w(int nx, int ny, int nz, int aligned)
+// nonzero if the x-sweep advectbyzx of this grid (one box, b(1) in place) reads the (rho, m_x)
+// side array when given: advect's choice of kernel
+static int advect_reads_w(int nx, int ny, int nz)
 {
-    (void)nx, (void)ny, (void)nz, (void)aligned;
-    return kV2;
+    AdvectArgs a{};  // any 16-byte aligned address stands in for the buffers
+    a.nx = nx;
+    a.ny = ny;
+    a.nz = nz;
+    a.ub = a.b1_src = a.w = reinterpret_cast<const void*>(uintptr_t(256));
+    A6Plan p6;
+    A4Plan p4;
+    A3Plan p3;
+    if (!kV2)
+        return 0;
+    if (plan_advect6(a, true, p6) || plan_advect4(a, true, p4))
+        return 1;
+    if (plan_advect3(nx, ny, nz, true, p3, 0, 2) && p3.C == 4)
+        return 1;
+    if (plan_advect3(nx, ny, nz, true, p3) || plan_advect(nx, ny, true).C)
+        return 0;
+    return rag_shape(nx, 2).C != 0 && !thread_per_cell_advect(nx, ny, nz, 1);
 }
 
-// nonzero if the transpose of this grid writes the side array when asked:
-// every FP32 kernel does
+// nonzero if the x-sweep fluidx of this grid is to write the side array (every FP32 kernel
+// does when asked): if the advectbyzx after it reads it
+static int fluidx_writes_w(int nx, int ny, int nz) { return advect_reads_w(nx, ny, nz); }
+
+// the same for the transpose of this grid, whose output the advectbyzx takes
 static int transpose_writes_w(int axis, int nx, int ny, int nz)
 {
-    (void)axis, (void)nx, (void)ny, (void)nz;
-    return kV2;
+    return axis == 1 ? advect_reads_w(ny, nx, nz) : advect_reads_w(nz, ny, nx);
 }
 
 // nonzero if the fused step's fluidx sweep along `axis` (1: y, 2: z) of this

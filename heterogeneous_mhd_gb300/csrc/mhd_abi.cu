@@ -751,8 +751,7 @@ static int enqueue_plain_step(mhd_ctx* c, double cfl)
     // the (rho, m_x) side array of a forward sweep's fluidx, read by the
     // advectbyzx launches right after it (8 instead of 20 bytes per cell)
     auto side = [&](int ax, int ay, int az) -> void* {
-        const bool al = ((size_t)ax * 5 * c->elem) % 16 == 0 && ((size_t)ax * 3 * c->elem) % 16 == 0;
-        return (c->W.p && c->ks->fluidx_writes_w(ax, ay, az, al ? 1 : 0)) ? c->W.p : nullptr;
+        return (c->W.p && c->ks->fluidx_writes_w(ax, ay, az)) ? c->W.p : nullptr;
     };
     MHD_TRY(op_finalize(c, c->part.p, c->clock.p, c->cfl_nparts, U0, B0, nx, ny, nz, cfl, 1));
     // x sweep
@@ -807,8 +806,7 @@ static int enqueue_fused_step(mhd_ctx* c, double cfl)
     // Every fluidx but the last writes the side array the advectbyzx after it
     // reads: rho and the momentum along that advectbyzx's sweep (1 m_x, 2 m_y,
     // 3 m_z), 8 instead of 20 bytes per cell.
-    const bool al = ((size_t)nx * 5 * c->elem) % 16 == 0 && ((size_t)nx * 3 * c->elem) % 16 == 0;
-    void* Wx = (c->W.p && c->ks->fluidx_writes_w(nx, ny, nz, al ? 1 : 0)) ? c->W.p : nullptr;
+    void* Wx = (c->W.p && c->ks->fluidx_writes_w(nx, ny, nz)) ? c->W.p : nullptr;
     void* Wy = (c->W.p && c->ks->sweep_writes_w(1, nx, ny, nz)) ? c->W.p : nullptr;
     void* Wz = (c->W.p && c->ks->sweep_writes_w(2, nx, ny, nz)) ? c->W.p : nullptr;
     MHD_TRY(op_finalize(c, c->part.p, c->clock.p, c->cfl_nparts, U0, B0, nx, ny, nz, cfl, 1));

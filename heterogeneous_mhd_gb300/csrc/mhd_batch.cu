@@ -368,7 +368,7 @@ static int enqueue_step(mhd_batch* b, double cfl)
         // the side array (classes with c.side): written by the forward fluidx launches
         // and the backward transposes, read by the advectbyzx after them, as in
         // the single-box plain step
-        void* const Wf = (c.side && b->ks->fluidx_writes_w(n, n, n, tma_ok(b, n))) ? c.W : nullptr;
+        void* const Wf = (c.side && b->ks->fluidx_writes_w(n, n, n)) ? c.W : nullptr;
         auto Wt = [&](int axis) -> void* {
             return (c.side && b->ks->transpose_writes_w(axis, n, n, n)) ? c.W : nullptr;
         };

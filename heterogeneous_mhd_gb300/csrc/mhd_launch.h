@@ -27,9 +27,10 @@ struct KernelSet {
     int (*fluidx_parts)(int nx, int ny, int nz, int aligned, int boxes);
     // nonzero if the sweeps along y and z of the fused step have kernels for this grid
     int (*fused_ok)(int nx, int ny, int nz);
-    // nonzero if the x-sweep fluidx of this grid writes the (rho, m_x) side array (FluidxArgs::w_out)
-    int (*fluidx_writes_w)(int nx, int ny, int nz, int aligned);
-    // nonzero if the transpose (axis 1 or 2) of this grid writes it (TransposeArgs::w_out)
+    // nonzero if the x-sweep fluidx of this grid is to write the (rho, m_x) side array
+    // (FluidxArgs::w_out): the advectbyzx after it reads it
+    int (*fluidx_writes_w)(int nx, int ny, int nz);
+    // nonzero if the transpose (axis 1 or 2) of this grid is to write it (TransposeArgs::w_out)
     int (*transpose_writes_w)(int axis, int nx, int ny, int nz);
     // nonzero if the fused step's fluidx sweep along `axis` (1: y) writes it
     int (*sweep_writes_w)(int axis, int nx, int ny, int nz);
