@@ -138,3 +138,21 @@ def test_fast_subnormal_pressure(shape, mhd, cuda, oracle32):
     d = gu.reshape(-1, 5).astype(np.float64) - uo.reshape(-1, 5)
     assert np.abs(d[:, 1:4]).max() <= 32 * 2.0 ** -149
     assert np.abs(d[:, 4]).max() <= 1e-5 * u[:, 4].max() and np.array_equal(gu[::5], uo[::5])
+
+
+@pytest.mark.parametrize("mode", ["f32", "f64"])
+@pytest.mark.parametrize("shape", ALL_SHAPES)
+def test_infinities_and_nan(shape, mode, mhd, cuda, oracle32, oracle64):
+    """One cell in fifty infinite, NaN or a signed zero: the bits of the reference (which
+    cells turn NaN or infinite, and all others)."""
+    o, dt = (oracle32, np.float32) if mode == "f32" else (oracle64, np.float64)
+    nc, rng = cells(shape, mode)
+    u, b, bin_ = (rng.standard_normal((nc, k)).astype(dt) for k in (5, 3, 3))
+    u[:, 0] = 2.0 ** rng.uniform(-3, 3, nc)
+    for x in (u, b, bin_):
+        m = rng.random(x.shape) < 0.02 / x.shape[1]
+        x[m] = rng.choice(np.array([np.inf, -np.inf, np.nan, 0.0, -0.0], dt), m.sum())
+    u, b, bin_ = u.ravel(), b.ravel(), bin_.ravel()
+    uo, bo = oracle_ops(o, u, b, bin_, shape, DT)
+    gu, gb = gpu_ops(mhd, cuda, u, b, bin_, shape, DT, exact=True, fp64=mode == "f64")
+    assert same_bits(gu, uo) and same_bits(gb, bo)
