@@ -336,3 +336,22 @@ def test_dgrad_pre_activations_on_a_channel_pair(n, clos, cuda):
         got.append(bf_np(y))
     assert clos.cl().mhd_cl_device_errors() == 0
     assert np.array_equal(got[0], got[1]) and np.abs(got[0]).max() > 0
+
+
+@pytest.mark.parametrize("nb,n", [(3, 40), (1, 56), (4, 64)])
+def test_wgrad_sets_of_several_tiles_vs_oracle(nb, n, clos, cuda):
+    """More tiles than partial sets (two per SM): 750 tiles in sets of 2 and 3, 686 likewise (the
+    last ones uneven), 4096 in sets of 13 and 14, each CTA working off two sets.  FP32 sums of
+    BF16 products: 1e-4 of the gradient's norm."""
+    torch = cuda
+    L, s = clos.cl(), clos.stream_ptr()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    a, dz = (torch.randn((nb, n, n, n, 32), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    scr = torch.empty(int(L.mhd_cl_wgrad_scratch(clos.WG_HID, nb, n)) // 4 + 1, dtype=torch.float32, device="cuda")
+    dw = torch.zeros(32 * 27 * 32, dtype=torch.float32, device="cuda")
+    assert L.mhd_cl_wgrad(clos.WG_HID, a.data_ptr(), dz.data_ptr(), scr.data_ptr(), dw.data_ptr(), nb, n, s) == 0
+    rows, av = dz.double().reshape(-1, 32).T, a.double()
+    ref = torch.stack([rows @ torch.roll(av, (1 - t // 9, 1 - (t // 3) % 3, 1 - t % 3), (1, 2, 3)).reshape(-1, 32)
+                       for t in range(27)], dim=1)
+    assert rel(dw.double().reshape(32, 27, 32).cpu().numpy(), ref.cpu().numpy()) < 1e-4
