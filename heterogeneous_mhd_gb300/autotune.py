@@ -63,12 +63,12 @@ def _time_kernel(ctx: Context, kernel: str, steps: int) -> float:
 
 
 def candidates(n: int):
-    """(knob settings) to try for fluidx and for advectbyzx on an n^3 grid."""
+    """(knob settings) to try for fluidx and for advectbyzx on an n^3 grid; {} is the planner's own."""
     fx = [{"fluidx.threads": t, "fluidx.cells": 4} for t in (64, 128, 256)]
     if n % 8 == 0 and 8 <= n // 8 <= 64 and (n // 8) & (n // 8 - 1) == 0:
         fx += [{"fluidx.threads": t, "fluidx.cells": 8} for t in (32, 64, 128, 256) if t >= n // 8]
-    adv = []
-    if n in (64, 128, 256):  # the warp-per-pencil kernel
+    adv = [{}]
+    if n in (64, 128, 256):  # the warp-per-pencil kernel (the planner's for 32, 96 and 192 too)
         for j in (2, 4):
             for k in (4, 8, 16, 32):
                 if n % j == 0 and n % k == 0:
@@ -135,8 +135,8 @@ def tune(n: int = 256, steps: int = 3, verbose: bool = False, save: bool = True)
 def batch_candidates(n: int):
     """Launch shapes to try for the boxes of edge n of a batch: the fluidx CTA
     width and the marching advectbyzx (the planner's kernel for classes
-    without the side array; classes with it, edges 96, 128 and 256, run the
-    warp-per-pencil kernel, against which the marching shapes are timed)."""
+    without the side array; classes with it, edges 32, 64, 96, 128, 192 and 256,
+    run the warp-per-pencil kernel, against which the marching shapes are timed)."""
     out = [{}]
     out += [{"fluidx.threads": t} for t in (128, 256)]
     t = n // 4
