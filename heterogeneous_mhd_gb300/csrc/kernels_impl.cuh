@@ -4,8 +4,9 @@
 // Each operator has a register-resident kernel for the common pencil lengths
 // (fluidx: n = 4T with T in {8..128} or 3T with T in {16..128}; advectbyzx:
 // n = 8T, T in {4..64} or 6T, T in {8..64}; transposes: bulk-TMA tiles of 32x32 or
-// 16x16 cells for edges that are multiples of 16) and a general kernel for
-// every other shape.  FP64 uses the general kernels.  The batch's work-list
+// 16x16 cells for edges that are multiples of 16); other FP32 lengths take the ragged
+// engine or one thread per cell, other transposes tiles of any edge.  FP64 takes one
+// thread per cell.  The batch's work-list
 // launches (one launch per operator over several size classes) are at the end.
 #include "mhd_advect2.cuh"
 #include "mhd_advect3.cuh"

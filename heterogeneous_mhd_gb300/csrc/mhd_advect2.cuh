@@ -116,7 +116,6 @@ __global__ void __launch_bounds__(512) k_advect2(AdvectArgs a)
 {
     after_previous();
     select_box(a, blockIdx.z);
-    using W = wide_t<R, EX>;
     constexpr int n = C * T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int P = a.P;

@@ -230,7 +230,6 @@ __device__ __forceinline__ void fluidx2_body(FluidxArgs a, const SweepMaps* tm, 
         __syncthreads();
     }
 
-    using W = wide_t<R, EX>;
 
     // ---- gather this thread's cells.  q and the cell-centred field are read
     // again from shared memory where they are needed later, which keeps them

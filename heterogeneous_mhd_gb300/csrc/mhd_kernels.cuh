@@ -525,14 +525,12 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
 {
     after_previous();
     select_box(a, blockIdx.z);
-    using W = wide_t<R, EX>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = a.nx, P = a.P;
     const int NR = advect_rows(P);
     const int items = NR * n;
     const int j0 = blockIdx.x * P, k = blockIdx.y;
     const int ny = a.ny, nz = a.nz;
-    const int km = (k == 0) ? nz - 1 : k - 1;
     const int kp = (k + 1 == nz) ? 0 : k + 1;
 
     R* VR = reinterpret_cast<R*>(smem_raw);  // raw face velocity, later the advected b
@@ -683,7 +681,6 @@ __global__ void __launch_bounds__(512) k_advect(AdvectArgs a)
         bo[cell * 3 + 1] = b2;
         bo[cell * 3 + 2] = b3;
     }
-    (void)km;
 }
 
 // -------------------------------------------------------------- transposes

@@ -80,7 +80,6 @@ __device__ __forceinline__ float rcp_ftz(float x)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double rcp_ftz(double x) { return 1.0 / x; }
 __device__ __forceinline__ float sqrt_ftz(float x)
 {
     float r;
@@ -100,7 +99,6 @@ __device__ __forceinline__ float mul_if_pos(float p, float x, float r)
         : "f"(p), "f"(x), "f"(r));
     return d;
 }
-__device__ __forceinline__ double mul_if_pos(double p, double x, double r) { return (p > 0.0) ? x * r : 0.0; }
 __device__ __forceinline__ float sub_if_pos(float p, float t, float x)
 {
     asm("{\n\t.reg .pred q;\n\tsetp.gt.f32 q, %1, 0f00000000;\n\t@q sub.rn.f32 %0, %0, %2;\n\t}"
@@ -108,7 +106,6 @@ __device__ __forceinline__ float sub_if_pos(float p, float t, float x)
         : "f"(p), "f"(x));
     return t;
 }
-__device__ __forceinline__ double sub_if_pos(double p, double t, double x) { return (p > 0.0) ? t - x : t; }
 
 // ------------------------------------------- EXACT in FP32 without FP64
 //
@@ -468,11 +465,12 @@ __device__ __forceinline__ R cfl_speed(const R q[5], const R f[3])
     }
 }
 
-// Per-cell steps of tvdb, shared by every advectbyzx kernel.  EXACT: the
-// reference's expressions (compiled without contraction).  FAST: every
-// rounding is explicit (__fadd_rn, __fmul_rn and __fmaf_rn are never
-// contracted), so all kernels compute the same bits whatever the compiler
-// does around the calls.
+// Per-cell steps of tvdb.  EXACT: the reference's values (compiled without contraction).
+// FAST: every rounding is explicit (__fadd_rn, __fmul_rn and __fmaf_rn are never
+// contracted), so k_advect2 to k_advect6 compute the same bits whatever the compiler
+// does around the calls.  k_advect and k_advect_rag, which share the other lengths and the
+// unaligned arrays, agree with each other: they divide for the face velocity and round the
+// half step's product by itself, so there the last bits differ from the others'.
 __device__ __forceinline__ float r_add(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double r_add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ float r_sub(float a, float b) { return __fsub_rn(a, b); }

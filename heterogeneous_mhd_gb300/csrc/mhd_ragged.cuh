@@ -1,8 +1,9 @@
-// fluidx and advectbyzx of the x sweep for pencils of any length (FP32): the
-// shapes that the fixed-length register engines (mhd_fluidx2.cuh,
-// mhd_advect2/3/6.cuh) were not laid out for (100, 72, 75, 33 cells), and
-// arrays that are not 16-byte aligned.  Both policies give the bits of the
-// one-thread-per-cell kernels that took these lengths before.
+// fluidx and advectbyzx of the x sweep (FP32) for pencil lengths that the fixed-length
+// register engines (mhd_fluidx2.cuh, mhd_advect2/3/6.cuh) were not laid out for (100,
+// 72, 75 cells), and for arrays that are not 16-byte aligned; short pencils and small
+// boxes of them take one thread per cell (thread_per_cell_fluidx, _advect in
+// kernels_impl.cuh).  EXACT gives the oracle's bits; FAST those of the one-thread-per-cell
+// kernels, which the tests pin.
 //
 // A pencil of n cells is held by T = ceil(n / C) threads with C (3, 4 or 5)
 // consecutive cells in registers; the last one holds the remaining L cells and,
@@ -11,8 +12,10 @@
 // instead of its cell 0, and the last thread sends its cell L-1 forwards.  A group of
 // G = 8, 16 or 32 W lanes holds a pencil (G >= T; the lanes past T repeat the
 // last thread and write nothing); C is the one with the fewest slots G C.
-// Up to 160 cells a pencil needs no barrier of its own: all exchanges are
-// shuffles.  Longer ones cross warps through shared memory and the CTA barrier.
+// Up to 160 cells fluidx needs no barrier of its own: all exchanges are shuffles.
+// Longer pencils cross warps through shared memory and the CTA barrier.  advectbyzx looks
+// two cells ahead, so its last thread holds two at least: 101, 131, 136, 141, 146, 151 and
+// 156 cells cross warps too, and a length one above a multiple of 60 has no such layout (k_advect).
 //
 // A pencil is staged by one bulk copy where it consists of aligned 16-byte
 // pieces, by 8- or 4-byte cp.async otherwise; the images are staged as well.  The kernels this
@@ -21,7 +24,7 @@
 // issue and latency (the boxes fit in L2).
 //
 // Measured (plain steps, with the transposes of mhd_kernels.cuh): four steps of
-// 100 x 72 x 72 in 1.67 ms before, 0.93 ms now; one step of 200 x 150 x 150 1.34 ms.
+// 100 x 72 x 72 in 1.67 ms with one thread per cell, 0.95 ms; one step of 200 x 150 x 150 1.34 ms.
 #pragma once
 #include "mhd_kernels.cuh"
 #include "mhd_launch.h"

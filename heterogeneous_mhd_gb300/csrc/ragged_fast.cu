@@ -64,7 +64,7 @@ cudaError_t fluidx_ragged(const FluidxArgs& in, bool exact, cudaStream_t s)
 // J pencils per CTA: five groups of 32 lanes or ten of 16 (the group of the
 // halo pencil is the price of a small J).  K planes: the K with the least waves of
 // CTAs x (K + 1.5), as a6_planes (four
-// steps of 100 x 72 x 72: 0.93 ms, 1.03 with the most planes that left 608 CTAs).
+// steps of 100 x 72 x 72: 0.95 ms, 1.05 with the most planes that left 608 CTAs).
 cudaError_t advect_ragged(const AdvectArgs& in, bool exact, cudaStream_t s)
 {
     AdvectArgs a = in;
