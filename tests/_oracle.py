@@ -2,7 +2,7 @@
 
 Two builds share one interface:
   * the restatement oracle/mhd_oracle.c -> oracle/_build/liboracle_{f32,f64}.so
-    (symbols orc_*), built everywhere, including the GPU box;
+    (symbols orc_*), built everywhere, including the GPU host;
   * the reference's own C/ sources -> oracle/_ref/libmhdref_{f32,f64}.so
     (symbols fluidx, advectbyzx, ...), built only where the reference
     sources exist.

@@ -169,3 +169,17 @@ def test_fast_ragged_bits_are_kept(case, mhd, cuda):
     run amplifies a last-bit change): digests made with them."""
     want = json.loads((GOLDEN / "fast_ragged.json").read_text())
     assert pinned_outputs(mhd, cuda, *case) == want["%dx%dx%d+%d" % case]
+
+
+@pytest.mark.parametrize("shape", [(20, 60, 60), (16, 80, 80), (12, 96, 96), (60, 20, 20), (40, 40, 40)])
+def test_steps_that_mix_both_kernels_vs_oracle(shape, mhd, cuda, oracle32):
+    """Plain steps whose fluidx takes one thread per cell and writes the side array for an
+    advectbyzx of the engine, in one sweep or another."""
+    u, b = mhd.init_vortex(*shape, seed=3)
+    ref = oracle32.strang(u, b, *shape, 2)
+    with mhd.Context(*shape, exact=True) as ctx:
+        ctx.set_state(u, b)
+        ctx.step(2, cfl=0.7)
+        gu, gb = ctx.get_state()
+        assert ctx.check() == mhd.MHD_OK
+    assert bitwise_equal(gu, ref[0]) and bitwise_equal(gb, ref[1])
