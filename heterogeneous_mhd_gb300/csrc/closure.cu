@@ -179,31 +179,37 @@ __global__ void __launch_bounds__(128) k_conv(const bf16* x, const bf16* w, cons
         const TileIdx t = tile_of(tile, n);
         __syncthreads();  // previous tile's readers are done with sx
         load_rows<CIN, KS>(sx, x, t, n);
-        float bs[2 * NT];  // the lane's channels' bias, read while the rows land
-        if constexpr (EPI != EPI_DGRAD) {
-#pragma unroll
-            for (int j = 0; j < 2 * NT; j++)
-                bs[j] = bias[(j / 2) * 8 + 2 * (lane & 3) + (j & 1)];
-        }
+        cp_async_wait_all();
+        __syncthreads();
+
+        // What the epilogue reads, before its first store (which could alias it): in the 3^3 kinds
+        // while the MMAs run, in the 1^3 kinds, whose CTAs per SM go by registers, after them.
         const size_t box0 = (size_t)t.box * n * n * n;
         auto voxel = [&](int i, int hr) {
             const int r = (lane >> 2) + 8 * hr;
             const int ty = 2 * i + (r >> 3), tx = r & 7;
             return box0 + ((size_t)(t.z0 + tz) * n + (t.y0 + ty)) * n + (t.x0 + tx);
         };
-        __nv_bfloat162 zp[MT][2][NT];  // and its pre-activations
-        if constexpr (EPI == EPI_DGRAD) {
+        float bs[2 * NT];               // the lane's channels' bias
+        __nv_bfloat162 zp[MT][2][NT];   // its pre-activations
+        auto read_ahead = [&] {
+            if constexpr (EPI != EPI_DGRAD) {
 #pragma unroll
-            for (int i = 0; i < MT; i++)
+                for (int j = 0; j < 2 * NT; j++)
+                    bs[j] = bias[(j / 2) * 8 + 2 * (lane & 3) + (j & 1)];
+            } else {
 #pragma unroll
-                for (int hr = 0; hr < 2; hr++)
+                for (int i = 0; i < MT; i++)
 #pragma unroll
-                    for (int j = 0; j < NT; j++)
-                        zp[i][hr][j] = *reinterpret_cast<const __nv_bfloat162*>(zprev + voxel(i, hr) * COUT + j * 8 +
-                                                                                2 * (lane & 3));
-        }
-        cp_async_wait_all();
-        __syncthreads();
+                    for (int hr = 0; hr < 2; hr++)
+#pragma unroll
+                        for (int j = 0; j < NT; j++)
+                            zp[i][hr][j] = *reinterpret_cast<const __nv_bfloat162*>(zprev + voxel(i, hr) * COUT +
+                                                                                    j * 8 + 2 * (lane & 3));
+            }
+        };
+        if constexpr (KS > 1)
+            read_ahead();
 
         float acc[MT][NT][4];
 #pragma unroll
@@ -250,6 +256,8 @@ __global__ void __launch_bounds__(128) k_conv(const bf16* x, const bf16* w, cons
         }
 
         // epilogue: rows lane/4 and lane/4 + 8 of each m-tile, channel pair 2*(lane%4)
+        if constexpr (KS == 1)
+            read_ahead();
 #pragma unroll
         for (int i = 0; i < MT; i++)
 #pragma unroll

@@ -141,17 +141,19 @@ static bool fluidx_range_ok(const FluidxArgs& a)
 
 // Where FP32 takes one thread per cell (k_fluidx, k_advect) instead of the ragged engine: short
 // pencils, which fill few of the engine's lanes, and small boxes, whose time is the latency of one
-// CTA's chain.  In both the CTAs must be filled (P pencils of n cells), or few.  Measured per launch
+// CTA's chain.  In both the CTAs must hold some pencils (a CTA costs 1.0 to 1.2 ns of a full
+// device and more with its warps, the engine 0.8 to 1.2 ns a pencil), or be few.  Measured per launch
 // (us, engine / one thread per cell; n x m x m cells, m = 32, 64, 128):
 //   fluidx      8: 6.8/4.1 7.3/4.2 15.7/5.4;  17: 7.9/5.2 8.6/6.1 18.2/13.8;  18: 6.5/5.1 7.3/6.2 12.1/13.8;
 //              20: 6.7/3.9 7.5/4.5 16.7/10.4;  31: 8.7/5.4 10.1/8.2 20.1/21.6;  40: 6.6/4.0 7.3/7.0 15/19
 //   advectbyzx  8: 9.3/6.2 9.8/6.2 17/9.4;  12: 6.6/6.1 7.2/6.7 12/11.9;  13: 9.6/5.1 11/6.1 19/12.6;
 //              24: 6.7/6.1 8.2/8.6 13/18.6;  31: 9.8/6.4 11.7/9.0 19/23;  40: 8.1/6.8 10.3/10.3 18/29
-// 131 pencils in a row (a prime: one to a CTA) of 12 cells, 127 planes: 13/21 and 12/27.
+// 131 pencils in a row (a prime: one to a CTA) of 12 cells, 127 planes: 13/21 and 12/27; 129 (three
+// to a CTA) of 8, 128 planes: 16.4/8.5 and 16.7/14.6.
 static bool cta_fills(int nx, int ny, int nz)
 {
     const int P = fluidx_pencils(nx, ny);  // advect_pencils is the same
-    return P * nx >= 64 || (long long)(ny / P) * nz <= 2048;
+    return P >= 3 || (P == 2 && nx <= 16) || (long long)(ny / P) * nz <= 2048;
 }
 
 constexpr long long kThreadPerCell = 200000;  // cells of a launch

@@ -224,12 +224,13 @@ __device__ __forceinline__ void rag_lds(const float* s, float (&d)[NF])
     }
 }
 
-// CTAs per SM that k_fluidx_rag is bounded to in FAST (0: as the compiler finds): the kinds whose
-// registers pass the next CTA's share (128 instead of 96, 79 instead of 72) without a bound and
-// hold in it without spills (pencils of 72 cells, four CTAs instead of five: 14.6 against 10.6 us).
+// CTAs per SM that k_fluidx_rag is bounded to in FAST (0: as the compiler finds): five (96
+// registers, C = 3: seven and 72) for the kinds that hold in it without spills but take 128 or 79
+// without a bound (pencils of 72 cells, four CTAs instead of five: 14.6 against 10.6 us); four
+// for <4, 3>, which takes 96 by itself and is faster with 128 (121 and 241 cells: 4 to 8%).
 constexpr int rag_fluidx_ctas(int C, int D)
 {
-    return C == 3 ? (D == 2 ? 7 : 0) : (C == 5 ? (D >= 3 ? 5 : 0) : (D % 3 ? 5 : 0));
+    return C == 3 ? (D == 2 ? 7 : 0) : (C == 5 ? (D >= 3 ? 5 : 0) : (D % 3 ? 5 : (D == 3 ? 4 : 0)));
 }
 
 // C/fluidx.c:19-102, C/tvd1.c:8-118, C/mhdflux.c:9-72; see fluidx2_body for the
